@@ -130,6 +130,70 @@ TRTC_FORCEINLINE bool spin_continue(uint32_t& spins, const uint32_t* err) {
     return true;
 }
 
+// ------------------------------------------------------------------ bulk copies
+// Bulk copy global -> shared by the tensor memory accelerator (cp.async.bulk, no
+// multicast), completing on a shared-memory mbarrier.  Both addresses 16-byte aligned, the
+// size a multiple of 16.  The copy's shared-memory writes do not use the SM's load/store
+// pipe.
+TRTC_FORCEINLINE uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+TRTC_FORCEINLINE void mbar_init(unsigned long long* bar, uint32_t arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(arrivals) : "memory");
+}
+// makes initialised barriers visible to the copy engine (async proxy)
+TRTC_FORCEINLINE void mbar_init_fence() {
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+}
+TRTC_FORCEINLINE void mbar_init_one(unsigned long long* bar) {
+    mbar_init(bar, 1u);
+    mbar_init_fence();
+}
+TRTC_FORCEINLINE void mbar_arrive(unsigned long long* bar) {
+    asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+}
+// one arrival that also announces `bytes` of bulk copies to wait for
+TRTC_FORCEINLINE void mbar_arrive_expect(unsigned long long* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
+                 : "memory");
+}
+TRTC_FORCEINLINE void bulk_load_g2s_more(void* sdst, const void* gsrc, uint32_t bytes, unsigned long long* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                     smem_u32(sdst)),
+                 "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+// a single copy: announced and issued
+TRTC_FORCEINLINE void bulk_load_g2s(void* sdst, const void* gsrc, uint32_t bytes, unsigned long long* bar) {
+    mbar_arrive_expect(bar, bytes);
+    bulk_load_g2s_more(sdst, gsrc, bytes, bar);
+}
+TRTC_FORCEINLINE bool mbar_try_wait(unsigned long long* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// has phase `parity` of the barrier completed?  (does not wait)
+TRTC_FORCEINLINE bool mbar_test(unsigned long long* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// bounded wait for phase `parity` of the barrier; false when the poll budget is spent
+TRTC_FORCEINLINE bool mbar_wait_bounded(unsigned long long* bar, uint32_t parity, const uint32_t* err) {
+    uint32_t spins = 0;
+    while (!mbar_try_wait(bar, parity))
+        if (!spin_continue(spins, err)) return false;
+    return true;
+}
+
 // ------------------------------------------------------------------ L2 eviction hints
 // 16-byte global loads/stores with an L2 eviction-priority policy (createpolicy, sm_80+).
 TRTC_FORCEINLINE unsigned long long l2_evict_last_policy() {

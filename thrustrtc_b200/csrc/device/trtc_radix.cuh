@@ -315,42 +315,6 @@ TRTC_FORCEINLINE void cp_async_elem(V* smem_dst, const V* gsrc) {
 }
 TRTC_FORCEINLINE void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Bulk copy global -> shared by the tensor memory accelerator (cp.async.bulk, no
-// multicast), completing on a shared-memory mbarrier.  Both addresses 16-byte aligned, the
-// size a multiple of 16.  The copy's shared-memory writes do not use the SM's load/store
-// pipe.
-TRTC_FORCEINLINE uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-TRTC_FORCEINLINE void mbar_init_one(unsigned long long* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(bar)) : "memory");
-    // make the initialised barrier visible to the copy engine (async proxy)
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-}
-TRTC_FORCEINLINE void bulk_load_g2s(void* sdst, const void* gsrc, uint32_t bytes, unsigned long long* bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                     smem_u32(sdst)),
-                 "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-TRTC_FORCEINLINE bool mbar_try_wait(unsigned long long* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// bounded wait for phase `parity` of the barrier; false when the poll budget is spent
-TRTC_FORCEINLINE bool mbar_wait_bounded(unsigned long long* bar, uint32_t parity, const uint32_t* err) {
-    uint32_t spins = 0;
-    while (!mbar_try_wait(bar, parity))
-        if (!spin_continue(spins, err)) return false;
-    return true;
-}
-
 // Digit of byte `pass` of the ordered key code: one byte permute on the 32-bit half that
 // holds it (sel = 0x4440 | byte index within the half).
 template <class K, bool DESC>

@@ -713,12 +713,87 @@ uint32_t TRTC_Partition_Stencil(DVVectorLike& vec, const DVVectorLike& stencil, 
     return partition_in_place(vec, &stencil, pred);
 }
 
-// reduce_by_key: segmented inclusive scan, then compaction of segment tails
-// (reduce.cpp:36-62); the tails are selected from the keys with the same predicate.
+// can a write to `w` reach what is read through `r`?  Known not to: two contiguous vectors with
+// disjoint byte ranges, a sink that drops what it is given, a view without memory.
+static bool cannot_overlap(const DVVectorLike& w, const DVVectorLike& r) {
+    if (w.name_view_cls().compare(0, 12, "DiscardView<") == 0) return true;
+    const char* wp = (const char*)w.contiguous_data();
+    if (!wp) return false;
+    const std::string& rc = r.name_view_cls();
+    if (rc.compare(0, 13, "ConstantView<") == 0 || rc.compare(0, 12, "CounterView<") == 0) return true;
+    const char* rp = (const char*)r.contiguous_data();
+    return rp && (wp + w.size() * w.elem_size() <= rp || rp + r.size() * r.elem_size() <= wp);
+}
+
+// reduce_by_key in one pass over the input (rbk_pipe_kernel), when the outputs cannot overlap
+// the inputs and keys and values are at most 16 bytes together (three tiles of 40 KB and the
+// staged results fill an SM's shared memory): tiles of 5120 elements of up to 8 bytes of key and
+// value, of 2560 up to 16.  20 and 10 elements per thread are 5 times 16 bytes of the widest
+// array: an odd number, so that the threads' 16-byte shared-memory loads do not share banks.
+// false: not this form (nothing was launched).
+static bool reduce_by_key_pipe(const DVVectorLike& key_in, const DVVectorLike& value_in, DVVectorLike& key_out,
+                               DVVectorLike& value_out, const Functor& pred, const Functor& op, uint32_t& count) {
+    const size_t n = key_in.size();
+    if (n >= 0xFFFFFFFFull) return false;
+    const DVVectorLike* ins[2] = {&key_in, &value_in};
+    const DVVectorLike* outs[2] = {&key_out, &value_out};
+    for (auto* o : outs)
+        for (auto* i : ins)
+            if (!cannot_overlap(*o, *i)) return false;
+    const std::string T = value_out.name_elem_cls();
+    Layout tl;
+    if (!layout_of(T, tl)) return false;
+    const size_t ks = key_in.elem_size(), vs = std::max(value_in.elem_size(), tl.size);
+    if (ks + vs > 16 || tl.align > 16) return false;
+    const int items = ks + vs <= 8 ? 20 : 10, stages = 3, groups = 2;
+    const size_t tile = (size_t)256 * items;
+    const size_t halo = (ks == 1 || ks == 2 || ks == 4 || ks == 8) ? 16 / ks : 1;
+    const size_t stage = round_up((tile + 2 * halo) * ks, 16) + round_up(tile * value_in.elem_size(), 16);
+    const size_t result = std::max(ks, tl.size) <= 4 ? 8 : 16;  // at most (RbkResult)
+    // the rest of an SM's shared memory holds staged results (at least a tile's twice over)
+    const size_t smem = 220 * 1024;
+    const size_t ring = ((smem - stages * stage) / result - tile) / 16 * 16;
+    const size_t tiles = (n + tile - 1) / tile;
+    uint32_t e8 = 0;
+    LookbackWs* w = lookback_ws(S(), tiles, tl.size, &e8);
+    if (!w) { count = (uint32_t)(-1); return true; }
+    trtc::LookbackState st;
+    st.flags = w->flags;
+    st.packed = w->packed;
+    st.agg = w->agg;
+    st.incl = w->incl;
+    st.tile_ctr = w->tile_ctr;
+    st.epoch8 = e8;
+    st.err = device_error_word();
+    st.result = w->result;
+    trtc::LookbackState st2 = st;
+    st2.packed = w->packed2;
+    const ViewArg kv = view_arg(key_in), vv = view_arg(value_in), ok = view_arg(key_out), ov = view_arg(value_out);
+    const std::string k = "trtc::rbk_pipe_kernel<" + kv.type + ", " + vv.type + ", " + ok.type + ", " + ov.type + ", " +
+                          T + ", " + pred.name_view_cls() + ", " + op.name_view_cls() + ", " + num(groups) + ", " + num(items) + ", " +
+                          num(stages) + ", " + num((long long)ring) + ">";
+    const size_t g = (size_t)sm_count();  // one of them the prefix CTA
+    unsigned long long cnt = 0;
+    const bool done = jit_run({"trtc_pipe.cuh"}, k, (unsigned)(g < tiles + 1 ? g : tiles + 1), (unsigned)(groups * 8 + 7) * 32,
+                              {kv.bytes, vv.bytes, ok.bytes, ov.bytes, pod_bytes<size_t>(n), pod_bytes<uint32_t>((uint32_t)tiles),
+                               pred.view(), op.view(), pod_bytes(st), pod_bytes(st2)},
+                              (unsigned)smem) &&
+                      TRTC_CUDA(cudaMemcpyAsync(&cnt, w->result, 8, cudaMemcpyDeviceToHost, S())) &&
+                      check_device_errors(S(), "reduce_by_key");
+    count = done ? to_u32(cnt) : (uint32_t)(-1);
+    return true;
+}
+
+// other forms: segmented inclusive scan, then compaction of segment tails (reduce.cpp:36-62);
+// the tails are selected from the keys with the same predicate.
 static uint32_t reduce_by_key_impl(const DVVectorLike& key_in, const DVVectorLike& value_in, DVVectorLike& key_out,
                                    DVVectorLike& value_out, const Functor& pred, const Functor& op) {
     const size_t n = key_in.size();
     if (n == 0) { set_error("reduce_by_key: empty input"); return (uint32_t)(-1); }
+    if (value_in.size() < n) { set_error("scan_by_key: fewer values than keys"); return (uint32_t)(-1); }
+    if (!ensure_device()) return (uint32_t)(-1);
+    uint32_t count = 0;
+    if (reduce_by_key_pipe(key_in, value_in, key_out, value_out, pred, op, count)) return count;
     DVVector scanned(value_out.name_elem_cls().c_str(), n);
     if (!scan_by_key_dispatch(key_in, value_in, scanned, pred, op, false, nullptr)) return (uint32_t)(-1);
     CompactSpec c;

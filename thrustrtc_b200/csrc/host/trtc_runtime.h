@@ -46,6 +46,7 @@ struct LookbackWs {
     void* agg = nullptr;
     void* incl = nullptr;
     unsigned long long* packed = nullptr;  // flag + value words for values of <= 4 bytes
+    unsigned long long* packed2 = nullptr; // a second set, for kernels with two look-backs
     unsigned long long* tile_ctr = nullptr;
     unsigned long long* result = nullptr;  // device scalar (count / total)
     size_t tiles_cap = 0;
