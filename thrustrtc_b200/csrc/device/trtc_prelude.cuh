@@ -194,6 +194,14 @@ TRTC_FORCEINLINE bool mbar_wait_bounded(unsigned long long* bar, uint32_t parity
     return true;
 }
 
+// ------------------------------------------------------------------ dependent launches
+// A kernel launched with programmatic stream serialisation starts while the kernel before it
+// drains; wait(): until that kernel has completed and its writes are visible, release(): the next
+// kernel may start once every CTA of this one has called it or left.  Without that launch
+// attribute both return at once.
+TRTC_FORCEINLINE void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+TRTC_FORCEINLINE void grid_dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------ L2 eviction hints
 // 16-byte global loads/stores with an L2 eviction-priority policy (createpolicy, sm_80+).
 TRTC_FORCEINLINE unsigned long long l2_evict_last_policy() {

@@ -5,15 +5,16 @@
 //   * hist kernel: one read of the keys builds the 256-bin histogram of every digit of the
 //     ordered key code (RadixKey<K>::ordered), flags NaNs, and clears the first look-back
 //     status array;
-//   * plan kernel: marks digits whose histogram has a bucket holding every key as no-ops
-//     (the reference's varying-bit mask, internal/radix_sort.cpp:11-45, at digit granularity),
-//     scans the histograms into bucket bases and picks the ping-pong buffer of every pass so
-//     the result lands in the caller's buffer without a host round trip;
+//   * plan (by the histogram's last CTA): marks digits whose histogram has a bucket holding
+//     every key as no-ops (the reference's varying-bit mask, internal/radix_sort.cpp:11-45, at
+//     digit granularity), scans the histograms into bucket bases and picks the ping-pong buffer
+//     of every pass so the result lands in the caller's buffer without a host round trip;
 //   * min-tree + count kernels (float/double, only when a NaN is present): the reference
 //     offsets keys by keys[TRTC_Min_Element], whose 256-wide tree (extrema.cpp:5-13 over
 //     internal/general_reduce.cpp:55-95) can select a non-minimum when NaNs sit in left slots;
 //     the sorted order is then a rotation, applied by the last digit pass's scatter;
-//   * one pass kernel per digit: a CTA takes tiles in launch order from an atomic counter,
+//   * short inputs: one CTA sorts all digits on chip in a single launch (radix_small_kernel);
+//   * one pass kernel per digit that moves data (the launches left over do nothing): a CTA takes tiles in launch order from an atomic counter,
 //     ranks its keys with warp multisplit (bit ballots), publishes per-digit counts,
 //     looks back across earlier tiles for its global offsets (decoupled look-back with
 //     release/acquire flags and bounded spins), stages the tile in shared memory in digit
@@ -27,18 +28,18 @@ namespace trtc {
 struct SortPlan {
     uint32_t active_mask;      // bit p: digit pass p moves data
     uint32_t num_active;
-    int32_t ordinal[8];        // running index of active pass p (selects the status array)
-    uint32_t src_sel[8];       // buffer set a pass reads: 0 caller, 1 temp A, 2 temp B
+    uint32_t digit[8];         // digit of the j-th launch, for j < num_active
+    uint32_t src_sel[8];       // buffer set the j-th launch reads: 0 caller, 1 temp A, 2 temp B
     uint32_t dst_sel[8];
-    int32_t last_pass;         // last active pass (applies the rotation)
     uint32_t copy_back;        // one active pass only: result sits in temp A
-    uint32_t base[8][256];     // exclusive bucket starts of every pass
+    uint32_t base[8][256];     // exclusive bucket starts of every digit
 };
 
 // Per-call control block; the host zeroes it (one memset) before every sort.
 struct SortCtrl {
     uint32_t hist[8][256];
     uint32_t tile_ctr[8];
+    uint32_t hist_done;             // CTAs that have added their histogram
     uint32_t nan_flag;
     uint32_t err;
     unsigned long long rot_count;   // keys ordered strictly below the selected minimum
@@ -94,6 +95,60 @@ __device__ inline uint32_t block_excl_scan_256(uint32_t v, uint32_t* s_wsum) {
 // lanes l and l+16 may share a word), whatever the key distribution.  Loads are 16-byte
 // vectors, UNROLL of them in flight per thread.
 template <class K> struct HistCopies { enum { V = RadixKey<K>::DIGITS > 4 ? 16 : 32 }; };
+
+// one CTA of BLOCK threads; s: 3 * BLOCK / 32 + D words of shared memory
+template <int D, int BLOCK>
+__device__ inline void radix_plan(SortCtrl* ctrl, size_t n, uint32_t* s) {
+    constexpr int G = BLOCK / 256;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, q = t >> 8;
+    uint32_t* s_wsum = s;
+    uint32_t* s_active = s + BLOCK / 32;
+    if (t < D) s_active[t] = 1u;
+    for (int p0 = 0; p0 < D; p0 += G) {
+        const int p = p0 + q;
+        const uint32_t c = p < D ? __ldcg(&ctrl->hist[p][t & 255]) : 0u;
+        uint32_t x = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
+        }
+        if (lane == 31) s_wsum[w] = x;
+        __syncthreads();
+        uint32_t pre = 0;
+        for (int i = w & ~7; i < w; i++) pre += s_wsum[i];
+        if (p < D) {
+            ctrl->plan.base[p][t & 255] = pre + x - c;
+            if (c == (uint32_t)n) s_active[p] = 0u;
+        }
+        __syncthreads();
+    }
+    if (t == 0) {
+        SortPlan& pl = ctrl->plan;
+        uint32_t mask = 0;
+        for (int p = 0; p < D; p++) mask |= s_active[p] << p;
+        const uint32_t a = (uint32_t)__popc(mask);
+        pl.active_mask = mask;
+        pl.num_active = a;
+        pl.copy_back = (a == 1) ? 1u : 0u;
+        uint32_t j = 0, cur = 0;
+        for (int p = 0; p < D; p++) {
+            if (!((mask >> p) & 1u)) continue;
+            uint32_t dst;
+            if (a == 1) dst = 1;
+            else if ((a & 1) == 0) dst = (j & 1) ? 0u : 1u;
+            else if (j == 0) dst = 1;
+            else if (j == 1) dst = 2;
+            else if (j == 2) dst = 0;
+            else dst = (j & 1) ? 1u : 0u;
+            pl.digit[j] = (uint32_t)p;
+            pl.src_sel[j] = cur;
+            pl.dst_sel[j] = dst;
+            cur = dst;
+            j++;
+        }
+    }
+}
 
 template <class K, bool DESC, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1) radix_hist_kernel(const typename RadixKey<K>::B* __restrict__ keys, size_t n,
@@ -159,51 +214,15 @@ __global__ void __launch_bounds__(BLOCK, 1) radix_hist_kernel(const typename Rad
         if (sum) atomicAdd(&ctrl->hist[0][0] + b, sum);
     }
     if (threadIdx.x == 0 && s_nan) atomicOr(&ctrl->nan_flag, 1u);
-}
-
-// ------------------------------------------------------------------ plan (1 block of 256)
-template <int D>
-__global__ void __launch_bounds__(256) radix_plan_kernel(SortCtrl* ctrl, size_t n) {
-    __shared__ uint32_t s_wsum[8];
-    __shared__ uint32_t s_active[8];
-    const int t = threadIdx.x;
-    for (int p = 0; p < D; p++) {
-        const uint32_t c = ctrl->hist[p][t];
-        const int full = __syncthreads_or(c == (uint32_t)n);
-        const uint32_t ex = block_excl_scan_256<256>(c, s_wsum);
-        ctrl->plan.base[p][t] = ex;
-        if (t == 0) s_active[p] = full ? 0u : 1u;
-    }
+    // the last CTA to add its histogram makes the plan (a launch of its own took 8 us of a short
+    // sort): 256 threads per digit, BLOCK / 256 digits at a time
+    __threadfence();
     __syncthreads();
-    if (t == 0) {
-        SortPlan& pl = ctrl->plan;
-        uint32_t mask = 0;
-        for (int p = 0; p < D; p++) mask |= s_active[p] << p;
-        const int a = __popc(mask);
-        pl.active_mask = mask;
-        pl.num_active = (uint32_t)a;
-        pl.copy_back = (a == 1) ? 1u : 0u;
-        pl.last_pass = -1;
-        int j = 0;
-        uint32_t cur = 0;
-        for (int p = 0; p < 8; p++) {
-            pl.ordinal[p] = 0; pl.src_sel[p] = 0; pl.dst_sel[p] = 0;
-            if (p >= D || !((mask >> p) & 1u)) continue;
-            uint32_t dst;
-            if (a == 1) dst = 1;
-            else if ((a & 1) == 0) dst = (j & 1) ? 0u : 1u;
-            else if (j == 0) dst = 1;
-            else if (j == 1) dst = 2;
-            else if (j == 2) dst = 0;
-            else dst = (j & 1) ? 1u : 0u;
-            pl.ordinal[p] = j;
-            pl.src_sel[p] = cur;
-            pl.dst_sel[p] = dst;
-            pl.last_pass = p;
-            cur = dst;
-            j++;
-        }
-    }
+    if (threadIdx.x == 0) s_nan = atomicAdd(&ctrl->hist_done, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!s_nan) return;
+    __threadfence();
+    radix_plan<D, BLOCK>(ctrl, n, s_hist);
 }
 
 // ------------------------------------------------------------------ Min_Element tree
@@ -390,6 +409,8 @@ constexpr bool radix_vbulk() {
             (size_t)TILE * sizeof(KB) >= radix_match_words<BLOCK>() * 4);
 }
 
+// ord: the launch's place among the digit passes; it runs the ord-th digit that moves data (none
+// past the last; after a single one, the second launch copies the result back).
 // HAS_VALS: move a 4- or 8-byte payload with the keys.  vals_from_index: the payload of the
 // first active pass is the element index (used to sort a permutation for odd value sizes).
 //
@@ -409,7 +430,7 @@ constexpr bool radix_vbulk() {
 //   5. write the tile out in bucket runs: consecutive threads write consecutive slots of a
 //      digit's run.
 template <class K, class V, bool HAS_VALS, bool DESC, int BLOCK, int ITEMS, class ST>
-__global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kernel(SortBufs bufs, size_t n, SortCtrl* ctrl, int pass,
+__global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kernel(SortBufs bufs, size_t n, SortCtrl* ctrl, int ord,
                                                            ST* status0, ST* status1, int vals_from_index,
                                                            uint32_t pf_tiles) {
     static_assert(BLOCK == 256, "one thread per digit");
@@ -424,7 +445,6 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     // element positions: 32-bit while n < 2^30 (ST = uint32_t), else 64-bit
     typedef typename conditional<(sizeof(ST) == 8), unsigned long long, uint32_t>::type IX;
     const SortPlan& plan = ctrl->plan;
-    if (!((plan.active_mask >> pass) & 1u)) return;
 
     extern __shared__ __align__(16) unsigned char smem[];
     KB* s_keys = reinterpret_cast<KB*>(smem);
@@ -439,12 +459,29 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     __shared__ __align__(8) unsigned long long s_vbar;  // completion of the bulk payload copy
     constexpr bool VB = radix_vbulk<KB, V, HAS_VALS, BLOCK, TILE>();
 
-    const int ord = plan.ordinal[pass];
+    // launched while the pass before drains (programmatic dependent launch)
+    grid_dependency_wait();
+    grid_dependency_release();
+    if ((uint32_t)ord >= plan.num_active) {
+        if (ord == 1 && plan.copy_back) {
+            // the only active pass left its result in temp A
+            const KB* sk = reinterpret_cast<const KB*>(bufs.keys[1]);
+            KB* dk = reinterpret_cast<KB*>(bufs.keys[0]);
+            const V* sv = reinterpret_cast<const V*>(bufs.vals[1]);
+            V* dv = reinterpret_cast<V*>(bufs.vals[0]);
+            for (size_t i = (size_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (size_t)gridDim.x * BLOCK) {
+                dk[i] = sk[i];
+                if (HAS_VALS) dv[i] = sv[i];
+            }
+        }
+        return;
+    }
+    const int pass = (int)plan.digit[ord];
     ST* st = (ord & 1) ? status1 : status0;
     ST* st_next = (ord & 1) ? status0 : status1;
     // buffer selection with selects (a runtime index into the parameter array would copy
     // it to local memory)
-    const uint32_t ss = plan.src_sel[pass], ds = plan.dst_sel[pass];
+    const uint32_t ss = plan.src_sel[ord], ds = plan.dst_sel[ord];
     const KB* __restrict__ src_k =
         reinterpret_cast<const KB*>(ss == 0 ? bufs.keys[0] : (ss == 1 ? bufs.keys[1] : bufs.keys[2]));
     KB* __restrict__ dst_k = reinterpret_cast<KB*>(ds == 0 ? bufs.keys[0] : (ds == 1 ? bufs.keys[1] : bufs.keys[2]));
@@ -455,17 +492,29 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     const bool hi = pass >= 4;
     const bool index_payload = HAS_VALS && vals_from_index && ord == 0;
     IX rot = 0;
-    if (FLOATKEY && pass == plan.last_pass && ctrl->rot_count) {
+    if (FLOATKEY && (uint32_t)ord + 1u == plan.num_active && ctrl->rot_count) {
         const unsigned long long k = ctrl->rot_count % n;
         rot = (IX)(DESC ? k : (k ? n - k : 0));
     }
 
-    if (threadIdx.x == 0) s_tile = atomicAdd(&ctrl->tile_ctr[ord], 1u);
+    // Resident CTAs take tiles in order until none is left (launches of one CTA per tile: 2^28 u32
+    // pairs 5.65 ms, 2^24 0.413 ms, and 15 us for a launch with nothing to do at 16,000 tiles;
+    // resident CTAs 5.55 and 0.398 ms, 2 us).  Keys-only passes draw the next ticket before they
+    // write a tile out (2^28 keys 4.49 -> 4.35 ms); pairs, which write twice as much meanwhile and
+    // so hold back the tiles that wait for theirs, after it (5.55 ms; before it 5.90 ms).
+    constexpr bool EARLY = !HAS_VALS;
+    const size_t tiles = (n + TILE - 1) / TILE;
+    uint32_t vphase = 0;
+    if (VB && threadIdx.x == 0) mbar_init_one(&s_vbar);
+    if (EARLY && threadIdx.x == 0) s_tile = atomicAdd(&ctrl->tile_ctr[ord], 1u);
+    for (;;) {
+    if (!EARLY && threadIdx.x == 0) s_tile = atomicAdd(&ctrl->tile_ctr[ord], 1u);
     for (int i = threadIdx.x; i < WARPS * 256; i += BLOCK) s_whist[i] = 0;
     if (TRTC_RADIX_MIXB < TRTC_RADIX_MIXP)
         for (int i = threadIdx.x; i < (int)radix_match_words<BLOCK>(); i += BLOCK) s_wmatch[i] = 0;
     __syncthreads();
     const size_t tile = s_tile;
+    if (tile >= tiles) return;
     st_next[tile * 256 + threadIdx.x] = 0;
 
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -486,7 +535,6 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     // uniform over the CTA: full tile, loaded payloads, 16-byte aligned source
     const bool vbulk = VB && full && !index_payload && ((reinterpret_cast<uintptr_t>(src_v + tile_base) & 15u) == 0);
     if (vbulk && threadIdx.x == 0) {
-        mbar_init_one(&s_vbar);
         bulk_load_g2s(s_vals, src_v + tile_base, (uint32_t)(TILE * sizeof(V)), &s_vbar);
     }
     // keys of this warp inside the tile (partial tiles only)
@@ -590,7 +638,7 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
             rank[i] += wh[radix_digit_sel<K, DESC>(keys[i], sel, hi)];
             s_keys[rank[i]] = keys[i];
         }
-        if (!mbar_wait_bounded(&s_vbar, 0u, bufs.err)) {
+        if (!mbar_wait_bounded(&s_vbar, vphase, bufs.err)) {
             report_error(bufs.err, TRTC_ERR_BULK_COPY_TIMEOUT);
             bad = true;
         }
@@ -665,6 +713,8 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
         return;
     }
 
+    uint32_t next = 0;
+    if (EARLY && threadIdx.x == 0 && gridDim.x < tiles) next = atomicAdd(&ctrl->tile_ctr[ord], 1u);
     // ---- 5. write out in bucket runs
     auto write_tile = [&](auto full_c) {
         constexpr bool FULL = decltype(full_c)::value;
@@ -686,9 +736,15 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     };
     if (full) write_tile(BoolC<true>());
     else write_tile(BoolC<false>());
+    if (gridDim.x >= tiles) return;  // a tile per CTA
+    vphase ^= vbulk ? 1u : 0u;
+    if (EARLY && threadIdx.x == 0) s_tile = next;
+    __syncthreads();
+    }
 }
 
-// single active pass: the result sits in temp A and is copied back to the caller's buffers
+// single active pass of single-digit keys (which have no second pass launch to do it): the result
+// sits in temp A and is copied back to the caller's buffers
 template <class K, class V, bool HAS_VALS>
 __global__ void radix_copyback_kernel(SortBufs bufs, size_t n, const SortCtrl* ctrl) {
     if (!ctrl->plan.copy_back) return;

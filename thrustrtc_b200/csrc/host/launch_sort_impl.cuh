@@ -35,6 +35,23 @@ static void set_smem_attr_once(F* kernel, size_t bytes) {
     }
 }
 
+// Launches a kernel that may start while the one before it on the stream drains (it waits for
+// that one's completion itself, grid_dependency_wait).
+template <class... P, class... A>
+static void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 // Runs the whole sort on stream s.  vals0 may be null (keys only).  vals_from_index: the
 // payload is the element index (vals0 then receives the sorting permutation).
 template <class K, class V, bool HAS_VALS, bool DESC, class ST, int ITEMS = SortTuning<K>::ITEMS>
@@ -83,9 +100,7 @@ static bool radix_sort_run(K* keys, V* vals0, size_t n, cudaStream_t s, int vals
         ktimer_mark("", s);
         hist_kernel<<<(unsigned)hgrid, HBLOCK, hsmem, s>>>((const KB*)keys, n, ctrl, (uint4*)st0, status_bytes / 16);
         ktimer_mark("radix_hist_kernel", s);
-        radix_plan_kernel<D><<<1, 256, 0, s>>>(ctrl, n);
-        ktimer_mark("radix_plan_kernel", s);
-        count_launch(2);
+        count_launch();
         if (FLOATKEY) {
             // the reference's Min_Element tree; only does work when a NaN was seen
             size_t m = n;
@@ -121,16 +136,23 @@ static bool radix_sort_run(K* keys, V* vals0, size_t n, cudaStream_t s, int vals
         // 5.739 ms without, 5.585 ms at 222 tiles, within 0.2 % from 148 to 444 tiles, slower
         // again past one wave of resident CTAs as the prefetched tiles crowd L2)
         const uint32_t pf = tile_prefetch_ahead((size_t)sms * 3 / 2);
+        static int per_sm = 0;
+        if (per_sm == 0 && (!TRTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel, BLOCK, smem)) || per_sm < 1))
+            per_sm = 1;
+        const size_t pgrid = (size_t)per_sm * sms < tiles ? (size_t)per_sm * sms : tiles;
         for (int p = 0; p < D; p++) {
-            pass_kernel<<<(unsigned)tiles, BLOCK, smem, s>>>(bufs, n, ctrl, p, (ST*)st0, (ST*)st1, vals_from_index, pf);
+            launch_dependent(pass_kernel, (unsigned)pgrid, BLOCK, smem, s, bufs, n, ctrl, p, (ST*)st0, (ST*)st1,
+                             vals_from_index, pf);
             ktimer_mark("radix_pass_kernel", s);
         }
         count_launch(D);
-        size_t cg = (n + 255) / 256;
-        if (cg > (size_t)sms * 8) cg = (size_t)sms * 8;
-        radix_copyback_kernel<K, V, HAS_VALS><<<(unsigned)cg, 256, 0, s>>>(bufs, n, ctrl);
-        count_launch();
-        ktimer_mark("radix_copyback_kernel", s);
+        if (D == 1) {
+            size_t cg = (n + 255) / 256;
+            if (cg > (size_t)sms * 8) cg = (size_t)sms * 8;
+            radix_copyback_kernel<K, V, HAS_VALS><<<(unsigned)cg, 256, 0, s>>>(bufs, n, ctrl);
+            count_launch();
+            ktimer_mark("radix_copyback_kernel", s);
+        }
         ok = TRTC_CUDA(cudaGetLastError());
     }
     for (int i = 0; i < 2; i++) { tmp_free(tv[i], s); tmp_free(ti[i], s); }
