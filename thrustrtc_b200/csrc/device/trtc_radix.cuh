@@ -743,6 +743,255 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     }
 }
 
+// ------------------------------------------------------------------ short inputs, one cluster
+// Sorts up to (cluster size) * blockDim.x * ITEMS keys (blockDim.x a multiple of 256) on chip, all
+// digits in one launch of one thread-block cluster: the keys (and payloads) stay in registers
+// between digits and change places through the CTAs' shared memory, CTA c holding slots
+// [c * per, (c + 1) * per).  Per digit: every warp ranks its keys with bit ballots and its own
+// digit counters, the CTAs tell each other their digit totals (stores into the others' shared
+// memory), each scans its counters digit-major / warp-minor behind what the totals say, and the
+// keys go to their slots, in whichever CTA; two cluster barriers per digit.  Digits in which all
+// keys agree are left out, as in the plan.  Slots past n hold keys of the highest digit in every
+// pass, so they stay behind the others.  Float keys with a NaN take the reference's Min_Element
+// rotation, as in the digit passes.  No global scratch, no other launch.
+// Bound by latency: 2 to 4 us per digit (the serial ranking, the barriers), where a launch per
+// digit with its look-back takes 8.  Measured shapes and times stand at radix_small_run.
+TRTC_FORCEINLINE uint32_t cluster_ctas() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r)); return r; }
+TRTC_FORCEINLINE uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+TRTC_FORCEINLINE void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of a shared-memory location (of this CTA's layout) in CTA `cta` of the cluster
+TRTC_FORCEINLINE uint32_t cluster_map(const void* p, uint32_t cta) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(cta));
+    return r;
+}
+template <class T> TRTC_FORCEINLINE void cluster_store(uint32_t addr, T v) {
+    if constexpr (sizeof(T) == 8) {
+        asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"((unsigned long long)v) : "memory");
+    } else if constexpr (sizeof(T) == 4) {
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"((uint32_t)v) : "memory");
+    } else if constexpr (sizeof(T) == 2) {
+        asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(addr), "h"((unsigned short)v) : "memory");
+    } else {
+        asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(addr), "r"((uint32_t)v) : "memory");
+    }
+}
+
+template <class KB, class V, bool HAS_VALS>
+constexpr size_t radix_small_smem(int block, int items) {
+    return (size_t)block * items * (sizeof(KB) + (HAS_VALS ? sizeof(V) : 0)) + (size_t)block / 32 * 256 * 4;
+}
+template <class K, class V, bool HAS_VALS, bool DESC, int ITEMS>
+__global__ void __launch_bounds__(1024, 1) radix_small_kernel(typename RadixKey<K>::B* keys, V* vals, uint32_t n,
+                                                              int vals_from_index) {
+    typedef RadixKey<K> RK;
+    typedef typename RK::B KB;
+    typedef typename RK::U U;
+    constexpr int D = RK::DIGITS;
+    constexpr bool FLOATKEY = is_same<K, float>::value || is_same<K, double>::value;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t threads = blockDim.x, warps = threads / 32, parts = threads / 256, per = threads * ITEMS;
+    const uint32_t ctas = cluster_ctas(), me = cluster_rank();
+    const bool solo = ctas == 1;  // one CTA: plain barriers and stores
+    auto sync_all = [&]() {
+        if (solo) __syncthreads();
+        else cluster_sync();
+    };
+    // slots by value size, so that every array is aligned: wide elements first
+    KB* s_keys = reinterpret_cast<KB*>(smem + (HAS_VALS && sizeof(V) > sizeof(KB) ? sizeof(V) * per : 0));
+    V* s_vals = reinterpret_cast<V*>(smem + (sizeof(V) > sizeof(KB) ? 0 : sizeof(KB) * per));
+    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + (sizeof(KB) + (HAS_VALS ? sizeof(V) : 0)) * per);  // [warps][256]
+    __shared__ uint32_t s_part[4][256], s_wsum[8];
+    __shared__ uint32_t s_total[16][256];  // every CTA's digit totals
+    __shared__ U s_or, s_varies[16];
+    __shared__ unsigned long long s_rot;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, ltm = lanemask_lt();
+    const uint32_t wbase = me * per + warp * 32u * ITEMS;  // the warp's first slot
+    KB k[ITEMS];
+    V v[HAS_VALS ? ITEMS : 1];
+    if (t == 0) { s_or = 0; s_rot = 0; }
+    __syncthreads();
+    // the bits in which keys differ, by comparison with the first key
+    const U ref = RK::ordered(keys[0]);
+    U o = 0;
+    bool nan = false;
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        const uint32_t p = wbase + (uint32_t)i * 32u + lane;
+        k[i] = p < n ? keys[p] : KB(0);
+        if (HAS_VALS) v[i] = p < n ? (vals_from_index ? (V)p : vals[p]) : V();
+        if (p < n) {
+            o |= RK::ordered(k[i]) ^ ref;
+            nan = nan || RK::is_nan(k[i]);
+        }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) o |= (U)__shfl_xor_sync(0xffffffffu, o, d);
+    if (lane == 0) atomicOr(&s_or, o);
+    // the same for the cluster; a NaN anywhere
+    const bool my_nan = FLOATKEY && __syncthreads_or(nan);
+    __syncthreads();
+    U varies = s_or;
+    bool any_nan = my_nan;
+    if (!solo) {
+        if (t == 0) s_wsum[0] = 0;
+        cluster_sync();  // every CTA runs: its shared memory may be written
+        if (t < ctas) {
+            cluster_store<U>(cluster_map(&s_varies[me], t), varies);
+            if (my_nan) cluster_store<uint32_t>(cluster_map(&s_wsum[0], t), 1u);
+        }
+        cluster_sync();
+        for (uint32_t c = 0; c < ctas; c++) varies |= s_varies[c];
+        any_nan = s_wsum[0] != 0;
+    }
+    uint32_t rot = 0;
+    if (FLOATKEY && any_nan) {
+        // the key that the reference's index tree selects (two rounds of 256-slot blocks), and the
+        // number of keys ordered below it; every CTA for itself, from the keys in place
+        __shared__ K s_tv[256];
+        __shared__ unsigned long long s_ti[256];
+        const uint32_t nb = (n + 255u) / 256u;
+        for (uint32_t b = warp; b < nb; b += warps) {
+            const uint32_t base = b * 256u, L = n - base < 256u ? n - base : 256u;
+            K rv;
+            unsigned long long ri;
+            min_tree_warp256<K>([&](uint32_t q, K& x, unsigned long long& ix) { x = RK::value(keys[base + q]); ix = base + q; },
+                                L, rv, ri);
+            if (lane == 0) { s_tv[b] = rv; s_ti[b] = ri; }
+        }
+        __syncthreads();
+        if (warp == 0 && nb > 1) {
+            K rv;
+            unsigned long long ri;
+            min_tree_warp256<K>([&](uint32_t q, K& x, unsigned long long& ix) { x = s_tv[q]; ix = s_ti[q]; }, nb, rv, ri);
+            __syncwarp();
+            if (lane == 0) s_ti[0] = ri;
+        }
+        __syncthreads();
+        const U tm = RK::ordered(keys[s_ti[0]]);
+        uint32_t below = 0;
+        for (uint32_t i = t; i < n; i += threads) below += RK::ordered(keys[i]) < tm ? 1u : 0u;
+        below = __reduce_add_sync(0xffffffffu, below);
+        if (lane == 0 && below) atomicAdd(&s_rot, (unsigned long long)below);
+        __syncthreads();
+        const uint32_t q = (uint32_t)(s_rot % n);
+        rot = DESC ? q : (q ? n - q : 0u);
+        sync_all();  // all have read the keys in place
+    }
+    __syncthreads();
+
+    uint32_t* wh = s_cnt + warp * 256u;
+#pragma unroll 1
+    for (int pass = 0; pass < D; pass++) {
+        if (((varies >> (8 * pass)) & 0xFFu) == 0) continue;
+        const uint32_t sel = 0x4440u | (uint32_t)(pass & 3);
+        const bool hi = pass >= 4;
+        for (uint32_t i = lane; i < 256u; i += 32u) wh[i] = 0;
+        __syncwarp();
+        uint32_t slot[ITEMS];
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const uint32_t d = wbase + (uint32_t)i * 32u + lane < n ? radix_digit_sel<K, DESC>(k[i], sel, hi) : 255u;
+            uint32_t peers = 0xffffffffu;
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                const uint32_t bal = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+                peers &= ((d >> b) & 1u) ? bal : ~bal;
+            }
+            const uint32_t before = wh[d];
+            slot[i] = before + (uint32_t)__popc(peers & ltm);
+            __syncwarp();
+            if ((peers & ltm) == 0) wh[d] = before + (uint32_t)__popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        // thread (part, digit): the digit's counters of 8 warps
+        const uint32_t part = t >> 8, dg = t & 255u;
+        uint32_t c8[8], sum = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            c8[w] = s_cnt[(part * 8u + w) * 256u + dg];
+            sum += c8[w];
+        }
+        s_part[part][dg] = sum;
+        __syncthreads();
+        uint32_t mine = 0;
+        if (t < 256) {
+            for (uint32_t q = 0; q < parts; q++) {
+                const uint32_t x = s_part[q][t];
+                s_part[q][t] = mine;
+                mine += x;
+            }
+            if (solo) s_total[0][t] = mine;
+            else
+                for (uint32_t c = 0; c < ctas; c++) cluster_store<uint32_t>(cluster_map(&s_total[me][t], c), mine);
+        }
+        sync_all();
+        if (t < 256) {
+            // the digit's keys in all CTAs, and in those before this one
+            uint32_t all = 0, before = 0;
+            for (uint32_t c = 0; c < ctas; c++) {
+                const uint32_t x = s_total[c][t];
+                if (c < me) before += x;
+                all += x;
+            }
+            uint32_t x = all;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= (uint32_t)d) x += y;
+            }
+            if (lane == 31) s_wsum[warp] = x;
+            asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
+            uint32_t pre = x - all + before;
+            for (uint32_t w = 0; w < warp; w++) pre += s_wsum[w];
+            for (uint32_t q = 0; q < parts; q++) s_part[q][t] += pre;
+        }
+        __syncthreads();
+        uint32_t run = s_part[part][dg];
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            s_cnt[(part * 8u + w) * 256u + dg] = run;
+            run += c8[w];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const uint32_t d = wbase + (uint32_t)i * 32u + lane < n ? radix_digit_sel<K, DESC>(k[i], sel, hi) : 255u;
+            const uint32_t p = slot[i] + wh[d];
+            if (solo) {
+                s_keys[p] = k[i];
+                if (HAS_VALS) s_vals[p] = v[i];
+            } else {
+                const uint32_t c = p / per, q = p % per;
+                cluster_store<KB>(cluster_map(s_keys + q, c), k[i]);
+                if (HAS_VALS) cluster_store<V>(cluster_map(s_vals + q, c), v[i]);
+            }
+        }
+        sync_all();
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const uint32_t q = warp * 32u * ITEMS + (uint32_t)i * 32u + lane;
+            k[i] = s_keys[q];
+            if (HAS_VALS) v[i] = s_vals[q];
+        }
+    }
+    // (every key equal: nothing moves, as in the reference; the permutation form still writes it)
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        uint32_t p = wbase + (uint32_t)i * 32u + lane;
+        if (p >= n) continue;
+        if (FLOATKEY) {
+            p += rot;
+            if (p >= n) p -= n;
+        }
+        keys[p] = k[i];
+        if (HAS_VALS) vals[p] = v[i];
+    }
+}
+
 // single active pass of single-digit keys (which have no second pass launch to do it): the result
 // sits in temp A and is copied back to the caller's buffers
 template <class K, class V, bool HAS_VALS>
@@ -762,7 +1011,7 @@ __global__ void radix_copyback_kernel(SortBufs bufs, size_t n, const SortCtrl* c
 // payloads of other sizes: values[i] = values_orig[perm[i]] through a temp copy
 static __global__ void radix_gather_bytes_kernel(const unsigned char* __restrict__ vals, unsigned char* __restrict__ tmp,
                                           const uint32_t* __restrict__ perm, size_t n, int esize, const SortCtrl* ctrl) {
-    if (ctrl->plan.num_active == 0) return;
+    if (ctrl && ctrl->plan.num_active == 0) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t s = perm[i];
         if (s >= n) continue;
@@ -771,7 +1020,7 @@ static __global__ void radix_gather_bytes_kernel(const unsigned char* __restrict
 }
 static __global__ void radix_copy_bytes_gated_kernel(const unsigned char* __restrict__ src, unsigned char* __restrict__ dst,
                                               size_t nbytes, const SortCtrl* ctrl) {
-    if (ctrl->plan.num_active == 0) return;
+    if (ctrl && ctrl->plan.num_active == 0) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nbytes; i += (size_t)gridDim.x * blockDim.x)
         dst[i] = src[i];
 }

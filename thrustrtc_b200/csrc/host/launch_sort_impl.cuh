@@ -161,6 +161,75 @@ static bool radix_sort_run(K* keys, V* vals0, size_t n, cudaStream_t s, int vals
     return ok;
 }
 
+// Up to this many keys one cluster sorts on chip in one launch.  B200, us per raw call (u32 pairs /
+// i64 keys with u32 values / u32 keys), cluster against the digit passes: 1024 keys 15 / 23 / 13
+// against 40 / 70 / 33, 8192 keys 24 / 40 / 20 against 40 / 78 / 35, 16384 30 / 50 / 26 against 43 /
+// 80 / 37, 32768 40 / 69 / 33 against 45 / 84 / 40; at 65536 keys (16 CTAs of 4096) 58 / 111 / 45
+// against 47 / 86 / 42.  CTAs of 256 threads x 4 keys are the fastest per key while 16 of them hold
+// the input (8192 keys on 8 x 512 threads 33 us, on 16 x 256 29 us); up to 2048 keys one CTA needs
+// no cluster barriers (2048 keys 17 us, on 8 CTAs 22 us).
+constexpr size_t RADIX_CLUSTER_N = 32768;
+// does the device place clusters of 16 CTAs of this kernel?  (a size above the portable 8)
+template <class F>
+static bool cluster16_fits(F* kernel, size_t smem) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 16;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const bool ok = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+constexpr int RADIX_SMALL_ITEMS = 4;
+template <class K, class V, bool HAS_VALS, bool DESC>
+static size_t radix_small_max() {
+    using namespace trtc;
+    static std::once_flag once;
+    static bool wide = false;
+    std::call_once(once, [&] {
+        auto kernel = radix_small_kernel<K, V, HAS_VALS, DESC, RADIX_SMALL_ITEMS>;
+        const size_t smem = radix_small_smem<typename RadixKey<K>::B, V, HAS_VALS>(512, RADIX_SMALL_ITEMS);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        wide = cluster16_fits(kernel, smem);
+    });
+    return wide ? RADIX_CLUSTER_N : RADIX_CLUSTER_N / 2;
+}
+template <class K, class V, bool HAS_VALS, bool DESC>
+static bool radix_small_run(K* keys, V* vals, size_t n, cudaStream_t s, int vals_from_index) {
+    using namespace trtc;
+    typedef typename RadixKey<K>::B KB;
+    constexpr int ITEMS = RADIX_SMALL_ITEMS;
+    auto kernel = radix_small_kernel<K, V, HAS_VALS, DESC, ITEMS>;
+    const bool wide = radix_small_max<K, V, HAS_VALS, DESC>() == RADIX_CLUSTER_N;
+    const int ctas = n <= 2048 ? 1 : n <= 8192 || !wide ? 8 : 16;
+    const int block = ((int)((n + (size_t)ctas * 1024 - 1) / ((size_t)ctas * 1024))) * 256;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = radix_small_smem<KB, V, HAS_VALS>(block, ITEMS);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = ctas > 1 ? 1 : 0;
+    ktimer_mark("", s);
+    const bool ok = TRTC_CUDA(cudaLaunchKernelEx(&cfg, kernel, (KB*)keys, vals, (uint32_t)n, vals_from_index));
+    count_launch();
+    ktimer_mark("radix_small_kernel", s);
+    return ok && TRTC_CUDA(cudaGetLastError());
+}
+
 template <class K, bool DESC>
 static bool radix_sort_dispatch(void* keys, void* vals, size_t vsize, size_t n, cudaStream_t s) {
     if (n >= (1ull << 32)) { set_error("sort: more than 2^32-1 keys"); return false; }
@@ -173,7 +242,9 @@ static bool radix_sort_dispatch(void* keys, void* vals, size_t vsize, size_t n, 
     constexpr int SMALL_ITEMS = sizeof(K) == 4 ? 8 : SortTuning<K>::ITEMS;
     const bool small = n <= TRTC_RADIX_SMALL_N;
 #define TRTC_SORT_RUN(V, HV, vp, fi)                                                                         \
-    (big ? radix_sort_run<K, V, HV, DESC, typename trtc::conditional<(sizeof(K) >= 4), unsigned long long, uint32_t>::type>( \
+    (n <= radix_small_max<K, V, HV, DESC>()                                                                 \
+         ? radix_small_run<K, V, HV, DESC>(k, (V*)(vp), n, s, fi)                                            \
+     : big ? radix_sort_run<K, V, HV, DESC, typename trtc::conditional<(sizeof(K) >= 4), unsigned long long, uint32_t>::type>( \
                k, (V*)(vp), n, s, fi)                                                                        \
          : small ? radix_sort_run<K, V, HV, DESC, uint32_t, SMALL_ITEMS>(k, (V*)(vp), n, s, fi)             \
                  : radix_sort_run<K, V, HV, DESC, uint32_t>(k, (V*)(vp), n, s, fi))
@@ -185,7 +256,10 @@ static bool radix_sort_dispatch(void* keys, void* vals, size_t vsize, size_t n, 
     unsigned char* tmpv = (unsigned char*)tmp_alloc(n * vsize, s);
     bool ok = perm && tmpv && TRTC_SORT_RUN(uint32_t, true, perm, 1);
     if (ok) {
-        trtc::SortCtrl* ctrl = (trtc::SortCtrl*)sort_ctrl_ws(s, sizeof(trtc::SortCtrl));
+        // (the gather is left out when the plan says that no key moves; the one-launch sort makes no
+        // plan, and its permutation is applied whatever it is)
+        const bool small_n = n <= radix_small_max<K, uint32_t, true, DESC>();
+        trtc::SortCtrl* ctrl = small_n ? nullptr : (trtc::SortCtrl*)sort_ctrl_ws(s, sizeof(trtc::SortCtrl));
         size_t g = (n + 255) / 256;
         if (g > (size_t)sm_count() * 8) g = (size_t)sm_count() * 8;
         trtc::radix_gather_bytes_kernel<<<(unsigned)g, 256, 0, s>>>((const unsigned char*)vals, tmpv, perm, n, (int)vsize, ctrl);
