@@ -115,18 +115,18 @@ bool scan_raw(int tc, int op, int mode, const void* in, void* out, size_t n, con
 
 // ---------------------------------------------------------------- reduce
 template <class T, class Op>
-static bool reduce_t(const T* in, size_t n, const T* init, void** result_dev, cudaStream_t s) {
+static bool reduce_t(const T* in, size_t n, const T* init, void** result_dev, void* to, cudaStream_t s) {
     constexpr int BLOCK = 256;
     const size_t nvec = n / VecWidth<T>::V;
     size_t grid = (nvec + BLOCK - 1) / BLOCK;
-    const size_t cap = (size_t)sm_count() * 8;
+    const size_t cap = (size_t)sm_count() * REDUCE_CTAS;
     if (grid > cap) grid = cap;
     if (grid < 1) grid = 1;
     LookbackWs* w = reduce_ws(s, grid, sizeof(T));
     if (!w) return false;
     ktimer_mark("", s);
     reduce_kernel<T, T, Op, Identity, false, BLOCK><<<(unsigned)grid, BLOCK, 0, s>>>(
-        in, n, Op(), Identity(), (T*)w->partials, w->partial_has, w->done_ctr, (T*)w->result, init ? 1 : 0,
+        in, n, Op(), Identity(), (T*)w->partials, w->partial_has, w->done_ctr, (T*)(to ? to : w->result), init ? 1 : 0,
         init ? *init : T());
     count_launch();
     ktimer_mark("reduce_kernel", s);
@@ -135,35 +135,46 @@ static bool reduce_t(const T* in, size_t n, const T* init, void** result_dev, cu
 }
 
 template <class T>
-static bool reduce_op(int op, const void* in, size_t n, const void* init, void** res, cudaStream_t s) {
+static bool reduce_op(int op, const void* in, size_t n, const void* init, void** res, void* to, cudaStream_t s) {
     switch (op) {
-        case OP_PLUS: return reduce_t<T, Plus>((const T*)in, n, (const T*)init, res, s);
-        case OP_MAX: return reduce_t<T, Maximum>((const T*)in, n, (const T*)init, res, s);
-        case OP_MIN: return reduce_t<T, Minimum>((const T*)in, n, (const T*)init, res, s);
+        case OP_PLUS: return reduce_t<T, Plus>((const T*)in, n, (const T*)init, res, to, s);
+        case OP_MAX: return reduce_t<T, Maximum>((const T*)in, n, (const T*)init, res, to, s);
+        case OP_MIN: return reduce_t<T, Minimum>((const T*)in, n, (const T*)init, res, to, s);
         default: set_error("reduce: unsupported operator"); return false;
     }
 }
 
-bool reduce_raw_async(int tc, int op, const void* in, size_t n, const void* init, void** res, cudaStream_t s) {
+// the result goes to `to` when given, else to the stream's device word, whose address is *res
+static bool reduce_to(int tc, int op, const void* in, size_t n, const void* init, void** res, void* to, cudaStream_t s) {
     if (n == 0 && !init) { set_error("reduce: empty input without an initial value"); return false; }
     switch (tc) {
-        case TC_I8: return reduce_op<int8_t>(op, in, n, init, res, s);
-        case TC_U8: return reduce_op<uint8_t>(op, in, n, init, res, s);
-        case TC_I16: return reduce_op<int16_t>(op, in, n, init, res, s);
-        case TC_U16: return reduce_op<uint16_t>(op, in, n, init, res, s);
-        case TC_I32: return reduce_op<int32_t>(op, in, n, init, res, s);
-        case TC_U32: return reduce_op<uint32_t>(op, in, n, init, res, s);
-        case TC_I64: return reduce_op<int64_t>(op, in, n, init, res, s);
-        case TC_U64: return reduce_op<uint64_t>(op, in, n, init, res, s);
-        case TC_F32: return reduce_op<float>(op, in, n, init, res, s);
-        case TC_F64: return reduce_op<double>(op, in, n, init, res, s);
+        case TC_I8: return reduce_op<int8_t>(op, in, n, init, res, to, s);
+        case TC_U8: return reduce_op<uint8_t>(op, in, n, init, res, to, s);
+        case TC_I16: return reduce_op<int16_t>(op, in, n, init, res, to, s);
+        case TC_U16: return reduce_op<uint16_t>(op, in, n, init, res, to, s);
+        case TC_I32: return reduce_op<int32_t>(op, in, n, init, res, to, s);
+        case TC_U32: return reduce_op<uint32_t>(op, in, n, init, res, to, s);
+        case TC_I64: return reduce_op<int64_t>(op, in, n, init, res, to, s);
+        case TC_U64: return reduce_op<uint64_t>(op, in, n, init, res, to, s);
+        case TC_F32: return reduce_op<float>(op, in, n, init, res, to, s);
+        case TC_F64: return reduce_op<double>(op, in, n, init, res, to, s);
         default: set_error("reduce: unsupported type"); return false;
     }
 }
 
+bool reduce_raw_async(int tc, int op, const void* in, size_t n, const void* init, void** res, cudaStream_t s) {
+    return reduce_to(tc, op, in, n, init, res, nullptr, s);
+}
+
 bool reduce_raw(int tc, int op, const void* in, size_t n, const void* init, void* result_host, cudaStream_t s) {
     void* rd = nullptr;
-    if (!reduce_raw_async(tc, op, in, n, init, &rd, s)) return false;
+    HostResult hr;
+    if (!reduce_to(tc, op, in, n, init, &rd, hr.dev(), s)) return false;
+    if (hr.dev()) {
+        if (!check_device_errors(s, "reduce")) return false;
+        hr.read(result_host, type_size(tc));
+        return true;
+    }
     return TRTC_CUDA(cudaMemcpyAsync(result_host, rd, type_size(tc), cudaMemcpyDeviceToHost, s)) &&
            check_device_errors(s, "reduce");
 }
@@ -294,6 +305,8 @@ static bool compact_t(const T* in, T* out, size_t n, const T* value, cudaStream_
     const size_t tiles = (n + TILE - 1) / TILE;
     LookbackState st;
     if (!fill_lookback(st, s, tiles, 8)) return false;
+    HostResult hr;
+    if (hr.dev()) st.result = hr.dev();
     VectorView<T> iv = make_view<T>(const_cast<T*>(in), n);
     VectorView<T> ov = make_view<T>(out, n);
     ktimer_mark("", s);
@@ -318,6 +331,11 @@ static bool compact_t(const T* in, T* out, size_t n, const T* value, cudaStream_
     count_launch();
     ktimer_mark("compact_kernel", s);
     if (!TRTC_CUDA(cudaGetLastError())) return false;
+    if (hr.dev()) {
+        if (!check_device_errors(s, "compaction")) return false;
+        hr.read(count, 8);
+        return true;
+    }
     return TRTC_CUDA(cudaMemcpyAsync(count, st.result, 8, cudaMemcpyDeviceToHost, s)) &&
            check_device_errors(s, "compaction");
 }

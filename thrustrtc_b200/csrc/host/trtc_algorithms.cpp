@@ -180,6 +180,29 @@ bool jit_copy(const ViewArg& in, const ViewArg& out, size_t n, size_t in_off = 0
                     pod_bytes<const unsigned long long*>(tail)});
 }
 
+// Reduction of a contiguous vector of a built-in type, each element through uop, under a built-in
+// (commutative) operator into the built-in type T: the grid-stride reduce kernel (B200, calls on
+// 16.8 M floats under a user's map: 52 us by the look-back scan kernel, 24 us by this one; 100 M
+// doubles 400 and 138 us).  `to`: where the result goes.
+bool jit_reduce(const DVVectorLike& in, const Functor& uop, const std::string& T, const Functor& op, const ViewBuf* init,
+                void* to) {
+    const size_t n = in.size();
+    const size_t vec = (size_t)vec_width(in.elem_size());
+    size_t grid = (n / vec + 255) / 256;
+    const size_t cap = (size_t)sm_count() * REDUCE_CTAS;
+    grid = grid > cap ? cap : grid < 1 ? 1 : grid;
+    Layout tl;
+    if (!layout_of(T, tl)) return false;
+    LookbackWs* w = reduce_ws(S(), grid, tl.size);
+    if (!w) return false;
+    const std::string k = "trtc::reduce_kernel<" + in.name_elem_cls() + ", " + T + ", " + op.name_view_cls() + ", " +
+                          uop.name_view_cls() + ", true, 256>";
+    return jit_run({"trtc_scan.cuh"}, k, (unsigned)grid, 256,
+                   {pod_bytes<void*>(in.contiguous_data()), pod_bytes<size_t>(n), op.view(), uop.view(),
+                    pod_bytes<void*>(w->partials), pod_bytes<void*>(w->partial_has), pod_bytes<void*>(w->done_ctr),
+                    pod_bytes<void*>(to), pod_bytes<int>(init ? 1 : 0), init ? *init : zero_of(T)});
+}
+
 // Scan-family kernel through NVRTC.  mode: 0 inclusive, 1 exclusive (init), 2 reduce,
 // 3 reduce with init; reductions leave their result in *result_dev.
 bool jit_scan(const DVVectorLike& in, const Functor* uop, const DVVectorLike* out, const std::string& T,
@@ -417,6 +440,17 @@ bool TRTC_Transform_Reduce(const DVVectorLike& vec, const Functor& unary_op, con
     const std::string T = init.name_view_cls();
     if (vec.size() == 0) { ret = init.view(); return true; }
     void* res = nullptr;
+    if (builtin_op_code(binary_op) >= 0 && type_code_of(T) >= 0 && type_code_of(vec.name_elem_cls()) >= 0 &&
+        vec.contiguous_data()) {
+        HostResult hr;
+        if (hr.dev()) {
+            const ViewBuf ini = init.view();
+            if (!jit_reduce(vec, unary_op, T, binary_op, &ini, hr.dev()) || !check_device_errors(S(), "reduce")) return false;
+            ret.resize(ini.size());
+            hr.read(ret.data(), ini.size());
+            return true;
+        }
+    }
     Layout tl;
     if (!layout_of(T, tl)) return false;
     if (!jit_scan(vec, &unary_op, nullptr, T, binary_op, 3, init.view(), &res)) return false;
@@ -559,6 +593,11 @@ unsigned long long run_compact(CompactSpec& c) {
     trtc::LookbackState lst;
     const bool c32 = n < (1ull << 32);  // 32-bit counts: flag and count in one look-back word
     if (!lookback_param(tiles, c32 ? 4 : 8, st, &lst)) return kFail;
+    HostResult hr;
+    if (hr.dev()) {
+        lst.result = hr.dev();
+        st = pod_bytes(lst);
+    }
     const std::string k = std::string(two_phase ? "trtc::compact2_kernel<" : "trtc::compact_kernel<") + num(c.mode) +
                           ", " + (c.partition ? "true" : "false") + ", " + (c.two ? "true" : "false") + ", " +
                           iv.type + ", " + sv.type + ", " + ptype + ", " + vtype + ", " + c.out.type + ", " +
@@ -579,9 +618,9 @@ unsigned long long run_compact(CompactSpec& c) {
     params.push_back(st);
     if (!jit_run({"trtc_compact.cuh"}, k, grid, 256, params)) return kFail;
     unsigned long long cnt = 0;
-    if (!TRTC_CUDA(cudaMemcpyAsync(&cnt, lst.result, 8, cudaMemcpyDeviceToHost, S())) ||
-        !check_device_errors(S(), "compaction"))
-        return kFail;
+    if (!hr.dev() && !TRTC_CUDA(cudaMemcpyAsync(&cnt, lst.result, 8, cudaMemcpyDeviceToHost, S()))) return kFail;
+    if (!check_device_errors(S(), "compaction")) return kFail;
+    if (hr.dev()) hr.read(&cnt, 8);
     return cnt;
 }
 
@@ -765,7 +804,8 @@ static bool reduce_by_key_pipe(const DVVectorLike& key_in, const DVVectorLike& v
     st.tile_ctr = w->tile_ctr;
     st.epoch8 = e8;
     st.err = device_error_word();
-    st.result = w->result;
+    HostResult hr;
+    st.result = hr.dev() ? hr.dev() : w->result;
     trtc::LookbackState st2 = st;
     st2.packed = w->packed2;
     const ViewArg kv = view_arg(key_in), vv = view_arg(value_in), ok = view_arg(key_out), ov = view_arg(value_out);
@@ -778,8 +818,9 @@ static bool reduce_by_key_pipe(const DVVectorLike& key_in, const DVVectorLike& v
                               {kv.bytes, vv.bytes, ok.bytes, ov.bytes, pod_bytes<size_t>(n), pod_bytes<uint32_t>((uint32_t)tiles),
                                pred.view(), op.view(), pod_bytes(st), pod_bytes(st2)},
                               (unsigned)smem) &&
-                      TRTC_CUDA(cudaMemcpyAsync(&cnt, w->result, 8, cudaMemcpyDeviceToHost, S())) &&
+                      (hr.dev() || TRTC_CUDA(cudaMemcpyAsync(&cnt, w->result, 8, cudaMemcpyDeviceToHost, S()))) &&
                       check_device_errors(S(), "reduce_by_key");
+    if (done && hr.dev()) hr.read(&cnt, 8);
     count = done ? to_u32(cnt) : (uint32_t)(-1);
     return true;
 }

@@ -9,6 +9,12 @@ namespace trtc_host {
 // compaction selector codes (same values as trtc::CompactMode)
 enum : int { COMPACT_NOT_EQUAL = 2, COMPACT_UNIQUE = 5 };
 
+// CTAs per SM of the reduce kernel: 4 x 256 threads with 16 loads each cover the memory latency, and
+// the last CTA folds half as many partials as with 8 (B200, per launch, float sums of 2^28 / 67 M /
+// 16.8 M / 4 M: 2 CTAs 191 / 56 / 21.8 / 12.1 us, 3: 166 / 50 / 20.7 / 11.9, 4: 160 / 48 / 20.7 / 11.8,
+// 8: 167 / 51 / 23.4 / 14.4)
+enum : int { REDUCE_CTAS = 4 };
+
 // radix sort of built-in key types; vals may be null; vsize = payload bytes per element
 bool sort_raw(int key_tc, void* keys, void* vals, size_t vsize, size_t n, bool desc, cudaStream_t s);
 bool sort_raw_narrow(int key_tc, void* keys, void* vals, size_t vsize, size_t n, bool desc, cudaStream_t s);

@@ -81,6 +81,24 @@ void tmp_free(void* p, cudaStream_t s);
 void* vector_alloc(size_t bytes);
 void vector_free(void* p);
 
+// A 16-byte host word that kernels write (mapped pinned memory): a call that returns a value to the
+// host has its kernel store it there, and after the call's synchronisation reads it without a copy
+// (the copy back into pageable memory and its own wait took 8 to 10 us of a short call).  One per
+// call under way, from a page of 256; dev() is null when none is free, and the caller then copies.
+class HostResult {
+public:
+    HostResult();
+    ~HostResult();
+    HostResult(const HostResult&) = delete;
+    HostResult& operator=(const HostResult&) = delete;
+    void* dev() const { return dev_; }
+    // after the stream is synchronised
+    void read(void* to, size_t bytes) const;
+private:
+    int slot_;
+    void* dev_;
+};
+
 int sm_count();
 
 }  // namespace trtc_host
