@@ -1281,6 +1281,7 @@ __global__ void __launch_bounds__(BLOCK, TRTC_SBK2_MINB(sizeof(T))) sbk2_kernel(
 #ifndef TRTC_REDUCE_UNROLL
 #define TRTC_REDUCE_UNROLL 16
 #endif
+template <int U> struct ReduceUnroll { static constexpr int value = U; };
 // Built-in commutative operators over contiguous input: 16-byte loads, VEC independent
 // per-thread accumulators (shorter FP accumulation chains), warp/block trees, one partial
 // per CTA, and the last CTA to finish folds the partials (no second launch).
@@ -1303,29 +1304,32 @@ __global__ void __launch_bounds__(BLOCK) reduce_kernel(const E* __restrict__ in,
     const size_t nvec = aligned ? n / VEC : 0;
     const size_t gtid = (size_t)blockIdx.x * BLOCK + threadIdx.x, gsz = (size_t)gridDim.x * BLOCK;
     size_t vi = gtid;
-    if (vi < nvec) {
-        union { uint4 q; E e[VEC]; } u;
-        u.q = reinterpret_cast<const uint4*>(in)[vi];
-#pragma unroll
-        for (int e = 0; e < VEC; e++) acc[e] = get(u.e[e]);
-        acc_h = true;
-        // U independent 16-byte loads in flight per thread
-        constexpr int U = TRTC_REDUCE_UNROLL;
-        for (vi += gsz; vi + (U - 1) * gsz < nvec; vi += U * gsz) {
+    // U independent 16-byte loads in flight per thread while that many are left to it, folded in
+    // order; the first load of all starts the accumulators
+    auto fold = [&](auto u_c) {
+        constexpr int U = decltype(u_c)::value;
+        for (; vi + (U - 1) * gsz < nvec; vi += U * gsz) {
             union { uint4 q; E e[VEC]; } w[U];
 #pragma unroll
             for (int r = 0; r < U; r++) w[r].q = reinterpret_cast<const uint4*>(in)[vi + r * gsz];
 #pragma unroll
-            for (int r = 0; r < U; r++)
+            for (int r = 0; r < U; r++) {
+                if (r == 0 && !acc_h) {
 #pragma unroll
-                for (int e = 0; e < VEC; e++) acc[e] = (T)op(acc[e], get(w[r].e[e]));
-        }
-        for (; vi < nvec; vi += gsz) {
-            u.q = reinterpret_cast<const uint4*>(in)[vi];
+                    for (int e = 0; e < VEC; e++) acc[e] = get(w[r].e[e]);
+                    acc_h = true;
+                } else {
 #pragma unroll
-            for (int e = 0; e < VEC; e++) acc[e] = (T)op(acc[e], get(u.e[e]));
+                    for (int e = 0; e < VEC; e++) acc[e] = (T)op(acc[e], get(w[r].e[e]));
+                }
+            }
         }
-    }
+    };
+    // (with single loads past the last 16, a thread of the 16.8 M float sum issued its 13 loads one
+    // after the other)
+    fold(ReduceUnroll<TRTC_REDUCE_UNROLL>());
+    fold(ReduceUnroll<4>());
+    fold(ReduceUnroll<1>());
     T a = acc[0];
     if (acc_h) {
 #pragma unroll
