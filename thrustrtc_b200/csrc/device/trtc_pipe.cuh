@@ -1,8 +1,9 @@
-// trtc_pipe.cuh -- persistent tile pipeline: reduce_by_key in one pass.
+// trtc_pipe.cuh -- persistent tile pipeline: reduce_by_key and compaction in one pass.
 //
 // The reference reduces by key with a segmented scan of every element, a scan of the tail
-// flags and a scatter (reduce.cpp:36-62).  Here a tile is read once, its segments are folded
-// on chip, and only the segments' keys and totals leave it.
+// flags and a scatter (reduce.cpp:36-62), and compacts with a flag scan and a scatter
+// (internal/general_copy_if.cpp:26-64).  Here a tile is read once, its segments are folded or its
+// elements selected on chip, and only the results leave it.
 //
 // A CTA runs five roles, handed from one to the next through mbarriers, so that none waits for
 // another's latency:
@@ -10,11 +11,11 @@
 //                     stages by TMA bulk copies;
 //   compute groups    (of 8 warps; tile k of the CTA is group k % G's) fold the tile, publish its
 //                     aggregates, give the input stage back and stage the results in a ring;
-//   two await warps   wait for what the tile needs from earlier tiles: the number of results
-//                     before it, and the running value of the segment that enters it;
+//   await warps       wait for what the tile needs from earlier tiles: the number of results
+//                     before it (and the running value of the segment that enters it);
 //   store warps       write the staged results at their final place (a tile each).
 // One CTA of the grid, the prefix CTA, scans what the tiles publish (half of its warps the counts,
-// half the running values) and answers every tile with what precedes it.  Tickets are drawn in
+// half the running values where there are any) and answers every tile with what precedes it.  Tickets are drawn in
 // order by running CTAs, so a tile only ever waits for tiles that are under way.
 //
 // Every wait is bounded: a role whose wait expires records the error and leaves, the others
@@ -239,7 +240,7 @@ template <int S> struct PipeBars {
     unsigned long long comp[PIPE_META];    // results staged (compute warps)
     unsigned long long pref[PIPE_META];    // prefixes known (await warps)
     unsigned long long done[PIPE_META];    // results written (store warp)
-    TRTC_FORCEINLINE void init() {
+    TRTC_FORCEINLINE void init(uint32_t await_warps) {
         for (int s = 0; s < S; s++) {
             mbar_init(&full[s], 1u);
             mbar_init(&empty[s], (uint32_t)PIPE_COMPUTE);
@@ -247,7 +248,7 @@ template <int S> struct PipeBars {
         for (int m = 0; m < PIPE_META; m++) {
             mbar_init(&agg[m], 1u);
             mbar_init(&comp[m], (uint32_t)PIPE_COMPUTE);
-            mbar_init(&pref[m], 2u);
+            mbar_init(&pref[m], await_warps);
             mbar_init(&done[m], 1u);
         }
         mbar_init_fence();
@@ -268,6 +269,60 @@ TRTC_FORCEINLINE void pipe_load_run(const T* s, T (&v)[ITEMS]) {
 #pragma unroll
         for (int i = 0; i < ITEMS; i++) v[i] = s[i];
     }
+}
+
+// The producer: draws tickets (the first, `t`, is already drawn; ticket t > 0 is tile t - 1) and has
+// issue(stage, tile, barrier) start the tile's bulk copies, or not (false: the compute group loads
+// the tile itself); after the last tile one stage per group carries the end mark.  A draw's round
+// trip (0.4 us) and the issue (0.3 us) bound a CTA's tile rate where a tile costs less than that.
+template <int G, int S, class Issue>
+TRTC_FORCEINLINE void pipe_produce(PipeBars<S>& bars, const LookbackState& st, uint32_t tiles, unsigned long long t,
+                                   uint32_t* s_tile, uint32_t* s_bulk, Issue issue) {
+    static_assert(S >= G, "the end reaches every group");
+    const unsigned long long last = (unsigned long long)tiles + gridDim.x - 1;
+    uint32_t ends = 0;
+    for (uint32_t k = 0;; k++) {
+        const uint32_t s = k % S;
+        if (k > 0 && ends == 0) t = atomicAdd(st.tile_ctr, 1ull);
+        if (ends == 0 && t == last) atomicExch(st.tile_ctr, 0ull);  // every ticket is taken
+        const bool ok = k < S || mbar_wait_bounded(&bars.empty[s], (k / S + 1u) & 1u, st.err);
+        if (!ok) {
+            report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
+            while (t <= (unsigned long long)tiles)
+                if ((t = atomicAdd(st.tile_ctr, 1ull)) == last) atomicExch(st.tile_ctr, 0ull);
+            // copies still under way write this CTA's shared memory
+            for (uint32_t q = k - S; q < k; q++) mbar_wait_bounded(&bars.full[q % S], (q / S) & 1u, nullptr);
+            return;
+        }
+        if (t > (unsigned long long)tiles) {
+            s_tile[s] = PIPE_END;
+            mbar_arrive(&bars.full[s]);
+            if (++ends == (uint32_t)G) return;
+            continue;
+        }
+        const uint32_t tile = (uint32_t)t - 1u;
+        s_tile[s] = tile;
+        s_bulk[s] = 0u;
+        if (!issue(s, tile, &bars.full[s])) mbar_arrive(&bars.full[s]);
+    }
+}
+// The store warps' wait for tile k of the CTA: 0 when it may be written, 1 at the end (m_last, the
+// CTA's number of tiles once known, is not above k), 2 when the wait ran out.
+template <int S>
+TRTC_FORCEINLINE int pipe_store_wait(PipeBars<S>& bars, uint32_t k, const uint32_t* m_last, uint32_t* err) {
+    const uint32_t m = k % PIPE_META, ph = (k / PIPE_META) & 1u;
+    uint32_t spins = 0;
+    int r = 0;
+    while (!mbar_try_wait(&bars.pref[m], ph)) {
+        if (*(volatile const uint32_t*)m_last <= k) { r = 1; break; }
+        if (!spin_continue(spins, err)) { r = 2; break; }
+    }
+    if (r == 0 && !mbar_wait_bounded(&bars.comp[m], ph, err)) r = 2;
+    if (__any_sync(0xffffffffu, r == 2)) {
+        if (lane_id() == 0) report_error(err, TRTC_ERR_LOOKBACK_TIMEOUT);
+        return 2;
+    }
+    return __any_sync(0xffffffffu, r == 1) ? 1 : 0;
 }
 
 // element sizes whose tiles are brought in by bulk copies (when contiguous and aligned)
@@ -321,7 +376,6 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
     constexpr uint32_t TILE = SM::TILE;
     constexpr int HALO = SM::HALO;
     static_assert(ITEMS < 32, "head mask");
-    static_assert(S >= G, "the end reaches every group");
     constexpr uint32_t OWN = (1u << ITEMS) - 1u;
     constexpr bool KTMA = ViewTraits<KV>::contiguous && PipeBulk<K>::value;
     constexpr bool VTMA = ViewTraits<VV>::contiguous && PipeBulk<E>::value;
@@ -344,12 +398,11 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
     auto skey = [&](uint32_t s) -> K* { return reinterpret_cast<K*>(pipe_smem + s * SM::STAGE) + HALO; };
     auto sval = [&](uint32_t s) -> E* { return reinterpret_cast<E*>(pipe_smem + s * SM::STAGE + SM::KEY_BYTES); };
     RbkResult<K, T>* ring = reinterpret_cast<RbkResult<K, T>*>(pipe_smem + SM::RING);
-    if (threadIdx.x == 0) bars.init();
+    if (threadIdx.x == 0) bars.init(2u);
     if (threadIdx.x == 0) m_last = 0xFFFFFFFFu;
     if (threadIdx.x < 2 * PIPE_META) m_stored[threadIdx.x] = 0;
     // tickets: the first one makes its CTA the prefix CTA (running before any tile can wait for it),
     // ticket t > 0 is tile t - 1; every other CTA draws until it holds one past the last tile
-    const unsigned long long last = (unsigned long long)tiles + gridDim.x - 1;
     if (threadIdx.x == 0) s_first = atomicAdd(st.tile_ctr, 1ull);
     __syncthreads();
     if (s_first == 0) {
@@ -545,18 +598,8 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
         // ------------------------------------------------------------ store
         const size_t ok_n = out_k.size(), ov_n = out_v.size();
         for (uint32_t k = warp - PIPE_COMPUTE * G;; k += PIPE_STORE) {
-            const uint32_t m = k % PIPE_META, ph = (k / PIPE_META) & 1u;
-            // (a warp whose next tile lies behind the end mark is told by m_last)
-            uint32_t spins = 0;
-            bool ok = true, stop = false;
-            while (!mbar_try_wait(&bars.pref[m], ph)) {
-                if (*(volatile uint32_t*)&m_last <= k) { stop = true; break; }
-                if (!spin_continue(spins, st.err)) { ok = false; break; }
-            }
-            stop = __any_sync(0xffffffffu, stop);
-            if (stop) return;
-            ok = ok && mbar_wait_bounded(&bars.comp[m], ph, st.err);
-            if (!__all_sync(0xffffffffu, ok)) { report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT); return; }
+            const uint32_t m = k % PIPE_META;
+            if (pipe_store_wait<S>(bars, k, &m_last, st.err)) return;
             const uint32_t cnt = m_cnt[m], start = m_start[m];
             const size_t base = m_base[m];
             const bool enters = m_open[m] && m_carry_h[m];  // the first result's segment began earlier
@@ -594,51 +637,242 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
             }
             return true;
         });
-    } else if (lane == 0) {
+    } else if (warp == PIPE_COMPUTE * G + PIPE_STORE + 2 && lane == 0) {
         // ------------------------------------------------------------ producer
         bool aligned = KTMA;
         if constexpr (KTMA) aligned = aligned && (reinterpret_cast<size_t>(keys._data) & 15u) == 0;
         if constexpr (VTMA) aligned = aligned && (reinterpret_cast<size_t>(vals._data) & 15u) == 0;
-        uint32_t ends = 0;
-        unsigned long long t = s_first;
-        for (uint32_t k = 0;; k++) {
-            const uint32_t s = k % S;
-            if (k > 0 && ends == 0) t = atomicAdd(st.tile_ctr, 1ull);
-            if (ends == 0 && t == last) atomicExch(st.tile_ctr, 0ull);  // every ticket is taken
-            const bool ok = k < S || mbar_wait_bounded(&bars.empty[s], (k / S + 1u) & 1u, st.err);
-            if (!ok) {
-                report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
-                while (t <= (unsigned long long)tiles)
-                    if ((t = atomicAdd(st.tile_ctr, 1ull)) == last) atomicExch(st.tile_ctr, 0ull);
-                // copies still under way write this CTA's shared memory
-                for (uint32_t q = k - S; q < k; q++) mbar_wait_bounded(&bars.full[q % S], (q / S) & 1u, nullptr);
-                return;
-            }
-            if (t > (unsigned long long)tiles) {
-                // the end, once for every group
-                s_tile[s] = PIPE_END;
-                mbar_arrive(&bars.full[s]);
-                if (++ends == (uint32_t)G) return;
-                continue;
-            }
-            const uint32_t tile = (uint32_t)t - 1u;
+        pipe_produce<G, S>(bars, st, tiles, s_first, s_tile, s_bulk, [&](uint32_t s, uint32_t tile, unsigned long long* full) -> bool {
             const size_t base = (size_t)tile * TILE;
-            const bool bulk = aligned && base + TILE + HALO <= n;
-            s_tile[s] = tile;
-            s_bulk[s] = bulk ? 1u : 0u;
-            if (!bulk) {
-                mbar_arrive(&bars.full[s]);
-                continue;
-            }
+            if (!aligned || base + TILE + HALO > n) return false;
             if constexpr (KTMA) {
                 const uint32_t lead = base > 0 ? (uint32_t)HALO : 0u;
                 const uint32_t kb = (TILE + HALO + lead) * (uint32_t)sizeof(K);
                 const uint32_t vb = VTMA ? TILE * (uint32_t)sizeof(E) : 0u;
-                mbar_arrive_expect(&bars.full[s], kb + vb);
-                bulk_load_g2s_more(skey(s) - (int)lead, keys._data + base - lead, kb, &bars.full[s]);
-                if constexpr (VTMA) bulk_load_g2s_more(sval(s), vals._data + base, vb, &bars.full[s]);
+                s_bulk[s] = 1u;
+                mbar_arrive_expect(full, kb + vb);
+                bulk_load_g2s_more(skey(s) - (int)lead, keys._data + base - lead, kb, full);
+                if constexpr (VTMA) bulk_load_g2s_more(sval(s), vals._data + base, vb, full);
+            }
+            return true;
+        });
+    }
+}
+
+// ---------------------------------------------------------------- compaction
+// Shared memory of the compaction pipeline: S input stages (the tile with a 16-byte lead, which
+// holds the element before it) and the ring of selected (and rejected) elements, as above.
+// Shapes: 3 groups, tiles of 20 KB (20 elements of 4 bytes, 10 of 8 per thread: 5 times 16 bytes, an odd
+// number, so that the threads' 16-byte shared-memory loads do not share banks), 3 stages, the rest of
+// 220 KB for the ring.  B200, 100 M int32, 50 / 90 / 100 % kept, us per launch: 3 groups, 20 elements, 3
+// stages 124 / 173 / 183, 4 stages 121 / 187 / 198 (a smaller ring), 2 groups 3 stages 129 / 174 / 186,
+// 2 groups 2 stages 136 / 167 / 175, 12 elements, 3 groups, 4 stages 154 / 169 / 175.  With few kept a
+// CTA's rate of tickets and issues bounds it (0.73 us per tile), with half kept HBM (5.0 TB/s), with all
+// kept the room for results that wait for their place (4 to 6 us from publication to answer).
+template <class E> struct CpipeShape {
+    static constexpr int G = 3, ITEMS = 80 / (int)sizeof(E), S = 3;
+    static constexpr int TILE = PIPE_COMPUTE * 32 * ITEMS;
+    static constexpr int RING = ((220 * 1024 - S * (TILE * (int)sizeof(E) + 16)) / (int)sizeof(E) - TILE) / 16 * 16;
+    static constexpr size_t SMEM = S * ((size_t)TILE * sizeof(E) + 16) + (size_t)(RING + TILE) * sizeof(E);
+};
+template <class E, int ITEMS, int S> struct CpipeSmem {
+    static constexpr int TILE = PIPE_COMPUTE * 32 * ITEMS;
+    static constexpr int LEAD = 16 / (int)sizeof(E);
+    static constexpr size_t STAGE = (size_t)(TILE + LEAD) * sizeof(E);
+    static constexpr size_t RING = S * STAGE;
+    static constexpr size_t bytes(size_t ring) { return RING + (ring + TILE) * sizeof(E); }
+};
+
+// Stable compaction of a contiguous array of 4- or 8-byte elements: elements selected by MODE
+// (CM_PRED, CM_NOT_EQUAL, CM_NOT_PRED, CM_UNIQUE, CM_UNIQUE_PRED) go to out, the rejected ones of
+// a partition to out_false, both in order; the number selected to *st.result.  The outputs do not
+// overlap the input.  C: ring size in elements.
+template <int MODE, bool PARTITION, class E, class Pred, class ValT, class OutV, class FalseV, int G, int ITEMS, int S, int C>
+__global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(const E* in, Pred pred, ValT value, OutV out,
+                                                                               FalseV out_false, size_t n, uint32_t tiles,
+                                                                               LookbackState st) {
+    typedef CpipeSmem<E, ITEMS, S> SM;
+    constexpr uint32_t TILE = SM::TILE;
+    constexpr bool NEIGH = MODE == CM_UNIQUE || MODE == CM_UNIQUE_PRED;
+    static_assert(ITEMS < 32 && C >= (int)TILE, "selection mask; a tile's elements fit the ring");
+    extern __shared__ __align__(16) unsigned char pipe_smem[];
+    __shared__ PipeBars<S> bars;
+    __shared__ uint32_t s_tile[S], s_bulk[S];
+    __shared__ uint32_t m_tile[PIPE_META], m_cnt[PIPE_META], m_all[PIPE_META], m_start[PIPE_META], m_base[PIPE_META];
+    __shared__ uint32_t m_end[2 * PIPE_META], m_stored[2 * PIPE_META];  // as in rbk_pipe_kernel
+    __shared__ uint32_t s_wcnt[2 * G][PIPE_COMPUTE];
+    __shared__ uint32_t m_last;
+    __shared__ unsigned long long s_first;
+
+    const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
+    auto stage = [&](uint32_t s) -> E* { return reinterpret_cast<E*>(pipe_smem + s * SM::STAGE) + SM::LEAD; };
+    E* ring = reinterpret_cast<E*>(pipe_smem + SM::RING);
+    if (threadIdx.x == 0) {
+        bars.init(1u);
+        m_last = 0xFFFFFFFFu;
+        s_first = atomicAdd(st.tile_ctr, 1ull);
+    }
+    if (threadIdx.x < 2 * PIPE_META) m_stored[threadIdx.x] = 0;
+    __syncthreads();
+    if (s_first == 0) {
+        constexpr int HALF = PipeShape<G>::WARPS / 2;
+        Plus plus;
+        if (warp < HALF)
+            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, tiles, plus, reinterpret_cast<unsigned long long*>(st.result), 0u, 1u);
+        return;
+    }
+    constexpr uint32_t GT = PIPE_COMPUTE * 32;  // threads of a group
+
+    if (warp < PIPE_COMPUTE * G) {
+        // ------------------------------------------------------------ compute
+        const uint32_t g = warp / PIPE_COMPUTE, gw = warp % PIPE_COMPUTE, gt = threadIdx.x % GT, bar = 1u + g;
+        const uint32_t t0 = gt * ITEMS;
+        uint32_t tail = 0, oldest = 0;
+        for (uint32_t k = g;; k += G) {
+            const uint32_t s = k % S, m = k % PIPE_META, b = (k / G % 2u) * G + g;
+            bool fail = !mbar_wait_bounded(&bars.full[s], (k / S) & 1u, st.err);
+            if (!fail && k >= (uint32_t)PIPE_META)
+                fail = !mbar_wait_bounded(&bars.done[m], (k / PIPE_META + 1u) & 1u, st.err);
+            if (fail) report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
+            if (pipe_any(bar, GT, fail)) return;
+            const uint32_t tile = s_tile[s];
+            if (gt == 0) m_tile[m] = tile;
+            if (tile == PIPE_END) {
+                if (gt == 0) {
+                    atomicMin(&m_last, k);
+                    mbar_arrive(&bars.agg[m]);
+                }
+                return;
+            }
+            const size_t base = (size_t)tile * TILE;
+            const uint32_t cnt = (n - base) < (size_t)TILE ? (uint32_t)(n - base) : TILE;
+            E* p = stage(s);
+            if (!s_bulk[s]) {
+                for (uint32_t i = gt; i < cnt; i += GT) p[i] = in[base + i];
+                if (NEIGH && gt == 0 && base > 0) p[-1] = in[base - 1];
+                // these writes come before a later bulk copy into the stage
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                pipe_sync(bar, GT);
+            }
+            E x[ITEMS];
+            pipe_load_run<E, ITEMS>(p + t0, x);
+            E before = E();
+            if constexpr (NEIGH) {
+                before = shfl_up_any(x[ITEMS - 1], 1);
+                if (lane == 0) before = p[(int)t0 - 1];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.empty[s]);
+            uint32_t sel = 0;
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++) {
+                bool f;
+                if constexpr (MODE == CM_PRED) f = (bool)pred(x[j]);
+                else if constexpr (MODE == CM_NOT_EQUAL) f = !(x[j] == value);
+                else if constexpr (MODE == CM_NOT_PRED) f = !(bool)pred(x[j]);
+                else if constexpr (MODE == CM_UNIQUE) f = x[j] != (j == 0 ? before : x[j > 0 ? j - 1 : 0]);
+                else f = !(bool)pred(x[j], j == 0 ? before : x[j > 0 ? j - 1 : 0]);
+                if (f) sel |= 1u << j;
+            }
+            if (NEIGH && tile == 0 && gt == 0) sel |= 1u;
+            const uint32_t left = cnt > t0 ? cnt - t0 : 0u;  // this thread's elements
+            if (left < (uint32_t)ITEMS) sel &= (1u << left) - 1u;
+            const uint32_t mine = (uint32_t)__popc(sel);
+            const uint32_t c = pipe_lane_sums<32>(mine);
+            if (lane == 31) s_wcnt[b][gw] = c;
+            pipe_sync(bar, GT);
+            const uint32_t wc = lane < (uint32_t)PIPE_COMPUTE ? s_wcnt[b][lane] : 0u;
+            const uint32_t wsum = pipe_lane_sums<PIPE_COMPUTE>(wc);
+            const uint32_t total = __shfl_sync(0xffffffffu, wsum, PIPE_COMPUTE - 1);
+            const uint32_t pos = __shfl_sync(0xffffffffu, wsum - wc, gw) + c - mine;  // selected before this thread's
+            const bool lead = gw == PIPE_COMPUTE - 1 && lane == 31;
+            if (lead) pipe_put<uint32_t>(st, tile, total, 1u);
+            const uint32_t need = PARTITION ? cnt : total;
+            uint32_t head = 0;
+            if (k > 0) {
+                const uint32_t pm = (k - 1u) % PIPE_META;
+                if (!mbar_wait_bounded(&bars.agg[pm], ((k - 1u) / PIPE_META) & 1u, st.err))
+                    report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
+                head = m_end[(k - 1u) % (2 * PIPE_META)];
+            }
+            if (k >= (uint32_t)PIPE_META && oldest <= k - PIPE_META) {
+                oldest = k - PIPE_META + 1u;
+                tail = m_end[(oldest - 1u) % (2 * PIPE_META)];
+            }
+            if (lead) {
+                m_cnt[m] = total;
+                m_all[m] = cnt;
+                m_start[m] = head % (uint32_t)C;
+                m_end[k % (2 * PIPE_META)] = head + need;
+                mbar_arrive(&bars.agg[m]);
+            }
+            for (uint32_t spins = 0; head + need - tail > (uint32_t)C;) {
+                if (*(volatile uint32_t*)&m_stored[oldest % (2 * PIPE_META)] == oldest + 1u) {
+                    tail = m_end[oldest % (2 * PIPE_META)];
+                    oldest++;
+                } else if (!spin_continue(spins, st.err)) {
+                    report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
+                    break;
+                }
+            }
+            E* r = ring + head % (uint32_t)C + pos;
+            E* q = ring + head % (uint32_t)C + total + (t0 - pos);  // rejected, behind the selected ones
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++) {
+                if ((sel >> j) & 1u) *r++ = x[j];
+                else if (PARTITION && j < (int)left) *q++ = x[j];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.comp[m]);
+        }
+    } else if (warp < PIPE_COMPUTE * G + PIPE_STORE) {
+        // ------------------------------------------------------------ store
+        const size_t out_n = out.size();
+        for (uint32_t k = warp - PIPE_COMPUTE * G;; k += PIPE_STORE) {
+            const uint32_t m = k % PIPE_META;
+            if (pipe_store_wait<S>(bars, k, &m_last, st.err)) return;
+            const uint32_t cnt = m_cnt[m], start = m_start[m];
+            const size_t base = m_base[m];
+            const size_t lim = base >= out_n ? 0 : out_n - base;
+            const uint32_t fit = cnt < lim ? cnt : (uint32_t)lim;
+            const E* r = ring + start;
+#pragma unroll 8
+            for (uint32_t i = lane; i < fit; i += 32) out[base + i] = r[i];
+            if constexpr (PARTITION) {
+                const size_t fbase = (size_t)m_tile[m] * TILE - base, false_n = out_false.size();
+                const uint32_t rej = m_all[m] - cnt;
+                const size_t flim = fbase >= false_n ? 0 : false_n - fbase;
+                const uint32_t ffit = rej < flim ? rej : (uint32_t)flim;
+                const E* f = r + cnt;
+#pragma unroll 8
+                for (uint32_t i = lane; i < ffit; i += 32) out_false[fbase + i] = f[i];
+            }
+            __syncwarp();
+            if (lane == 0) {
+                __threadfence_block();
+                *(volatile uint32_t*)&m_stored[k % (2 * PIPE_META)] = k + 1u;
+                mbar_arrive(&bars.done[m]);
             }
         }
+    } else if (warp == PIPE_COMPUTE * G + PIPE_STORE) {
+        // ------------------------------------------------------------ await
+        pipe_await_slots(bars.agg, bars.pref, m_tile, st.err, [&](uint32_t m, uint32_t tile) -> bool {
+            uint32_t pre = 0;
+            if (!pipe_answer<uint32_t>(st, tile, pre)) return false;
+            m_base[m] = pre;
+            return true;
+        });
+    } else if (warp == PIPE_COMPUTE * G + PIPE_STORE + 1 && lane == 0) {
+        // ------------------------------------------------------------ producer
+        const bool aligned = (reinterpret_cast<size_t>(in) & 15u) == 0;
+        pipe_produce<G, S>(bars, st, tiles, s_first, s_tile, s_bulk, [&](uint32_t s, uint32_t tile, unsigned long long* full) -> bool {
+            const size_t base = (size_t)tile * TILE;
+            if (!aligned || base + TILE > n) return false;
+            const uint32_t lead = NEIGH && base > 0 ? (uint32_t)SM::LEAD : 0u;
+            s_bulk[s] = 1u;
+            bulk_load_g2s(stage(s) - (int)lead, in + base - lead, (TILE + lead) * (uint32_t)sizeof(E), full);
+            return true;
+        });
     }
 }
 

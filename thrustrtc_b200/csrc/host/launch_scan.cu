@@ -2,7 +2,7 @@
 // kernels for the built-in element types and operators (Plus, Maximum, Minimum, EqualTo).
 #include "trtc_launch.h"
 #include "trtc_runtime.h"
-#include "../device/trtc_compact.cuh"
+#include "../device/trtc_pipe.cuh"
 
 namespace trtc_host {
 
@@ -295,6 +295,33 @@ static bool compact_t(const T* in, T* out, size_t n, const T* value, cudaStream_
             return ok;
         }
         (void)cudaGetLastError();  // the failed allocation must not fail the launch check below
+    }
+    if constexpr ((sizeof(T) == 4 || sizeof(T) == 8) && sizeof(CT) == 4) {
+        if (disjoint) {
+            // 4- and 8-byte elements: the tile pipeline (B200, 100 M int32: remove of few 202 -> 195 us
+            // per call, unique of runs of 32 157 -> 106, of 2 177 -> 129; int64 unique 339 -> 189)
+            typedef CpipeShape<T> SH;
+            const size_t tiles = (n + SH::TILE - 1) / SH::TILE;
+            LookbackState st;
+            if (!fill_lookback(st, s, tiles, 4)) return false;
+            HostResult hr;
+            if (hr.dev()) st.result = hr.dev();
+            auto kernel = compact_pipe_kernel<MODE, false, T, EqualTo, T, VectorView<T>, Nothing, SH::G, SH::ITEMS, SH::S, SH::RING>;
+            static const bool ready =
+                TRTC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::SMEM));
+            if (!ready) return false;
+            const size_t g = (size_t)sm_count();  // one of them the prefix CTA
+            ktimer_mark("", s);
+            kernel<<<(unsigned)(g < tiles + 1 ? g : tiles + 1), PipeShape<SH::G>::THREADS, SH::SMEM, s>>>(
+                in, EqualTo(), value ? *value : T(), make_view<T>(out, n), Nothing(), n, (uint32_t)tiles, st);
+            count_launch();
+            ktimer_mark("compact_kernel", s);
+            if (!TRTC_CUDA(cudaGetLastError())) return false;
+            if (!hr.dev() && !TRTC_CUDA(cudaMemcpyAsync(count, st.result, 8, cudaMemcpyDeviceToHost, s))) return false;
+            if (!check_device_errors(s, "compaction")) return false;
+            if (hr.dev()) hr.read(count, 8);
+            return true;
+        }
     }
     // the vector path (4-byte elements: remove's element-wise test, unique's neighbour test)
     // takes TRTC_COMPACT2_ITEMS; other widths take TRTC_COMPACT2_GENERIC_ITEMS

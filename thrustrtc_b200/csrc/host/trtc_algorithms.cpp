@@ -577,6 +577,39 @@ unsigned long long run_compact(CompactSpec& c) {
         }
         (void)cudaGetLastError();  // the failed allocation must not fail a later launch check
     }
+    // one array of 4- or 8-byte elements, outputs disjoint: the tile pipeline.  B200, calls on 100 M
+    // int32, compact2_kernel against it: 5 / 50 / 90 % kept 154 / 167 / 191 us against 110 / 130 / 186;
+    // partition 267 against 208, of int64 327 against 390: partitions of 8-byte elements keep the former
+    // (their results fill the ring whatever is selected)
+    const bool pipe_mode = c.mode == CM_PRED || c.mode == CM_NOT_EQUAL || c.mode == CM_NOT_PRED || c.mode == CM_UNIQUE ||
+                           c.mode == CM_UNIQUE_PRED;
+    const size_t es = c.in->elem_size();
+    if (two_phase && pipe_mode && !c.two && !c.stencil && (es == 4 || (es == 8 && !c.partition)) && c.in->contiguous_data() &&
+        n < 0xFFFFFFFFull) {
+        const int items = 80 / (int)es, stages = 3;  // (CpipeShape)
+        const size_t tile = (size_t)256 * items, tiles = (n + tile - 1) / tile;
+        const size_t stage = tile * es + 16;
+        const size_t ring = ((220 * 1024 - stages * stage) / es - tile) / 16 * 16;
+        ViewBuf st;
+        trtc::LookbackState lst;
+        if (!lookback_param(tiles, 4, st, &lst)) return kFail;
+        HostResult hr;
+        if (hr.dev()) lst.result = hr.dev();
+        const std::string k = "trtc::compact_pipe_kernel<" + num(c.mode) + ", " + (c.partition ? "true" : "false") + ", " +
+                              c.in->name_elem_cls() + ", " + ptype + ", " + vtype + ", " + c.out.type + ", " +
+                              c.out_false.type + ", 3, " + num(items) + ", " + num(stages) + ", " + num((long long)ring) + ">";
+        const size_t g = (size_t)sm_count();  // one of them the prefix CTA
+        if (!jit_run({"trtc_pipe.cuh"}, k, (unsigned)(g < tiles + 1 ? g : tiles + 1), (3 * 8 + 7) * 32,
+                     {pod_bytes<void*>(c.in->contiguous_data()), pbytes, vbytes, c.out.bytes, c.out_false.bytes,
+                      pod_bytes<size_t>(n), pod_bytes<uint32_t>((uint32_t)tiles), pod_bytes(lst)},
+                     (unsigned)(stages * stage + (ring + tile) * es)))
+            return kFail;
+        unsigned long long cnt = 0;
+        if (!hr.dev() && !TRTC_CUDA(cudaMemcpyAsync(&cnt, lst.result, 8, cudaMemcpyDeviceToHost, S()))) return kFail;
+        if (!check_device_errors(S(), "compaction")) return kFail;
+        if (hr.dev()) hr.read(&cnt, 8);
+        return cnt;
+    }
     // the 16-byte vector path (contiguous 4-byte input and output: element-wise tests of one
     // array, or neighbour tests with an optional second array) takes 32 items per thread; the
     // other two-phase forms (views, other widths, stencils, partitions) hold their rows in
