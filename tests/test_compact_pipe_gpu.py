@@ -1,4 +1,4 @@
-"""The compaction pipeline at the edges of its tiles and over several turns of its ring: every
+"""The compaction pipeline at the edges of its range and tiles and over many turns of its ring: every
 selection mode it takes, 4- and 8-byte elements, kept shares from none to all, partitions,
 unaligned ranges, outputs that are too short, against numpy."""
 import numpy as np
@@ -14,7 +14,9 @@ def trtc(cuda):
     return t
 
 
-SIZES = [1, 19, 20, 21, 2559, 2560, 2561, 5119, 5120, 5121, 5124, 10240, 40_001, 5120 * 148 * 4 + 3]
+# the pipeline starts at 2^22 elements; tiles of 5120 4-byte and 2560 8-byte elements
+EDGE = -(-(1 << 22) // 5120) * 5120
+SIZES = [1, 4097, (1 << 22) - 1, 1 << 22, EDGE - 1, EDGE, EDGE + 1, EDGE + 19, EDGE + 2559, EDGE + 2561, 5120 * 148 * 40 + 9]
 
 
 def check(trtc, got, out, want):
@@ -62,9 +64,9 @@ def test_modes(trtc, n, dtype):
 @pytest.mark.parametrize("off", [1, 2, 3])
 @pytest.mark.parametrize("dtype", [np.int32, np.int64])
 def test_unaligned_ranges_and_in_place(trtc, off, dtype):
-    n = 33_333
+    n = (1 << 22) + 33_333
     rng = np.random.default_rng(off)
-    x = np.sort(rng.integers(0, 3000, n + off)).astype(dtype)
+    x = np.sort(rng.integers(0, 400_000, n + off)).astype(dtype)
     d = trtc.device_vector_from_numpy(x)
     v = x[off:]
     o = dest(trtc, n, dtype)
@@ -77,9 +79,9 @@ def test_unaligned_ranges_and_in_place(trtc, off, dtype):
 
 
 def test_short_outputs_are_filled_to_their_end(trtc):
-    x = np.arange(50_000, dtype=np.int32)
+    x = np.arange(5_000_000, dtype=np.int32)
     d = trtc.device_vector_from_numpy(x)
     even = trtc.Functor({}, ["x"], "        return (x & 1) == 0;\n")
     o, r = dest(trtc, 7001, np.int32), dest(trtc, 333, np.int32)
-    assert trtc.Copy_If(d, o, even) == 25_000 and o.to_host().tobytes() == x[::2][:7001].tobytes()
-    assert trtc.Partition_Copy(d, o, r, even) == 25_000 and r.to_host().tobytes() == x[1::2][:333].tobytes()
+    assert trtc.Copy_If(d, o, even) == 2_500_000 and o.to_host().tobytes() == x[::2][:7001].tobytes()
+    assert trtc.Partition_Copy(d, o, r, even) == 2_500_000 and r.to_host().tobytes() == x[1::2][:333].tobytes()

@@ -37,7 +37,7 @@ def check(trtc, k, v, dk, dv, ufunc=np.add, op=None, pred=None, off=0):
     assert vo.to_host()[c] == 77  # nothing written behind the last segment
 
 
-SIZES = [1, 2, 19, 20, 5119, 5120, 5121, 5124, 5128, 10240, 15361, 40_001, 5120 * 4 * 300 + 5]
+SIZES = [1, 2, 19, 20, 5119, 5120, 5121, 5124, 5128, 10240, 15361, 40_001, 5120 * 4 * 300 + 5, 5120 * 148 * 40 + 9]
 
 
 @pytest.mark.parametrize("n", SIZES)

@@ -122,10 +122,11 @@ TRTC_FORCEINLINE void pipe_await_slots(unsigned long long* agg, unsigned long lo
 // of their own.  With a decoupled look-back by every tile instead (300 to 1200 warps polling up
 // to 128 words a round, the frontier moving one window per round trip) the tiles of 50 M elements
 // took 150 to 210 us where they take 88 us without any wait for prefixes.
-// WARPS warps from warp0 on run one stream of values; bar: a barrier of their own.
+// WARPS warps from warp0 on run one stream of values, published in st, answered in `answers` (the same
+// words, or others); bar: a barrier of their own.
 template <class T, class Op, bool SEG, int WARPS>
-__device__ void pipe_prefix_scan(const LookbackState& st, uint32_t tiles, Op& op, unsigned long long* result,
-                                 uint32_t warp0, uint32_t bar) {
+__device__ void pipe_prefix_scan(const LookbackState& st, const LookbackState& answers, uint32_t tiles, Op& op,
+                                 unsigned long long* result, uint32_t warp0, uint32_t bar) {
     static_assert(WARPS <= 16, "one scan of 16 warps");
     __shared__ uint32_t s_lead[32], s_hd[32], s_has[32], s_taken;
     __shared__ T s_v[32], s_total;
@@ -203,7 +204,7 @@ __device__ void pipe_prefix_scan(const LookbackState& st, uint32_t tiles, Op& op
                 p = ((hm & (le >> 1)) != 0u || !ph) ? ve : (T)op(p, ve);
                 ph = true;
             }
-            pipe_put<T>(st, j, p, ph ? 6u : 2u);
+            pipe_put<T>(answers, j, p, ph ? 6u : 2u);
         }
         if (taken) {
             run = s_total;
@@ -233,18 +234,20 @@ TRTC_FORCEINLINE uint32_t pipe_lane_sums(uint32_t v) {
     return v;
 }
 
-template <int S> struct PipeBars {
-    unsigned long long full[S];            // input stage loaded (producer, and its bulk copies)
+// A parity wait tells a phase from its neighbours only, so a waiter has to be at most one phase behind
+// or ahead.  Stage k % S is loaded for other groups in between where S is not a multiple of G, and
+// loads complete in any order: "loaded" has a barrier per k % L, L a multiple of both, each always the
+// same group's, which waits for every phase of it.
+template <int S, int L> struct PipeBars {
+    unsigned long long full[L];            // tile loaded (producer, and its bulk copies)
     unsigned long long empty[S];           // input stage read (compute warps)
     unsigned long long agg[PIPE_META];     // aggregates published (compute)
     unsigned long long comp[PIPE_META];    // results staged (compute warps)
     unsigned long long pref[PIPE_META];    // prefixes known (await warps)
     unsigned long long done[PIPE_META];    // results written (store warp)
     TRTC_FORCEINLINE void init(uint32_t await_warps) {
-        for (int s = 0; s < S; s++) {
-            mbar_init(&full[s], 1u);
-            mbar_init(&empty[s], (uint32_t)PIPE_COMPUTE);
-        }
+        for (int s = 0; s < L; s++) mbar_init(&full[s], 1u);
+        for (int s = 0; s < S; s++) mbar_init(&empty[s], (uint32_t)PIPE_COMPUTE);
         for (int m = 0; m < PIPE_META; m++) {
             mbar_init(&agg[m], 1u);
             mbar_init(&comp[m], (uint32_t)PIPE_COMPUTE);
@@ -275,8 +278,8 @@ TRTC_FORCEINLINE void pipe_load_run(const T* s, T (&v)[ITEMS]) {
 // issue(stage, tile, barrier) start the tile's bulk copies, or not (false: the compute group loads
 // the tile itself); after the last tile one stage per group carries the end mark.  A draw's round
 // trip (0.4 us) and the issue (0.3 us) bound a CTA's tile rate where a tile costs less than that.
-template <int G, int S, class Issue>
-TRTC_FORCEINLINE void pipe_produce(PipeBars<S>& bars, const LookbackState& st, uint32_t tiles, unsigned long long t,
+template <int G, int S, int L, class Issue>
+TRTC_FORCEINLINE void pipe_produce(PipeBars<S, L>& bars, const LookbackState& st, uint32_t tiles, unsigned long long t,
                                    uint32_t* s_tile, uint32_t* s_bulk, Issue issue) {
     static_assert(S >= G, "the end reaches every group");
     const unsigned long long last = (unsigned long long)tiles + gridDim.x - 1;
@@ -291,25 +294,25 @@ TRTC_FORCEINLINE void pipe_produce(PipeBars<S>& bars, const LookbackState& st, u
             while (t <= (unsigned long long)tiles)
                 if ((t = atomicAdd(st.tile_ctr, 1ull)) == last) atomicExch(st.tile_ctr, 0ull);
             // copies still under way write this CTA's shared memory
-            for (uint32_t q = k - S; q < k; q++) mbar_wait_bounded(&bars.full[q % S], (q / S) & 1u, nullptr);
+            for (uint32_t q = k - S; q < k; q++) mbar_wait_bounded(&bars.full[q % L], (q / L) & 1u, nullptr);
             return;
         }
         if (t > (unsigned long long)tiles) {
             s_tile[s] = PIPE_END;
-            mbar_arrive(&bars.full[s]);
+            mbar_arrive(&bars.full[k % L]);
             if (++ends == (uint32_t)G) return;
             continue;
         }
         const uint32_t tile = (uint32_t)t - 1u;
         s_tile[s] = tile;
         s_bulk[s] = 0u;
-        if (!issue(s, tile, &bars.full[s])) mbar_arrive(&bars.full[s]);
+        if (!issue(s, tile, &bars.full[k % L])) mbar_arrive(&bars.full[k % L]);
     }
 }
 // The store warps' wait for tile k of the CTA: 0 when it may be written, 1 at the end (m_last, the
 // CTA's number of tiles once known, is not above k), 2 when the wait ran out.
-template <int S>
-TRTC_FORCEINLINE int pipe_store_wait(PipeBars<S>& bars, uint32_t k, const uint32_t* m_last, uint32_t* err) {
+template <int S, int L>
+TRTC_FORCEINLINE int pipe_store_wait(PipeBars<S, L>& bars, uint32_t k, const uint32_t* m_last, uint32_t* err) {
     const uint32_t m = k % PIPE_META, ph = (k / PIPE_META) & 1u;
     uint32_t spins = 0;
     int r = 0;
@@ -380,7 +383,8 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
     constexpr bool KTMA = ViewTraits<KV>::contiguous && PipeBulk<K>::value;
     constexpr bool VTMA = ViewTraits<VV>::contiguous && PipeBulk<E>::value;
     extern __shared__ __align__(16) unsigned char pipe_smem[];
-    __shared__ PipeBars<S> bars;
+    constexpr int L = S % G == 0 ? S : S * G;
+    __shared__ PipeBars<S, L> bars;
     __shared__ uint32_t s_tile[S], s_bulk[S];                     // per input stage
     __shared__ uint32_t m_tile[PIPE_META], m_cnt[PIPE_META];      // per tile under way: its results,
     __shared__ uint32_t m_start[PIPE_META], m_base[PIPE_META];    // their place in the ring and in the output,
@@ -409,9 +413,9 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
         constexpr int HALF = PipeShape<G>::WARPS / 2;
         Plus plus;
         if (warp < HALF)
-            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, tiles, plus, reinterpret_cast<unsigned long long*>(st.result), 0u, 1u);
+            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, st, tiles, plus, reinterpret_cast<unsigned long long*>(st.result), 0u, 1u);
         else if (warp < 2 * HALF)
-            pipe_prefix_scan<T, Op, true, HALF>(st2, tiles, op, nullptr, HALF, 2u);
+            pipe_prefix_scan<T, Op, true, HALF>(st2, st2, tiles, op, nullptr, HALF, 2u);
         return;
     }
     constexpr uint32_t GT = PIPE_COMPUTE * 32;  // threads of a group
@@ -423,7 +427,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
         uint32_t tail = 0, oldest = 0;  // ring position of the first tile not known to be stored
         for (uint32_t k = g;; k += G) {
             const uint32_t s = k % S, m = k % PIPE_META, b = (k / G % 2u) * G + g;
-            bool fail = !mbar_wait_bounded(&bars.full[s], (k / S) & 1u, st.err);
+            bool fail = !mbar_wait_bounded(&bars.full[k % L], (k / L) & 1u, st.err);
             // the tile's bookkeeping slot is free again
             if (!fail && k >= (uint32_t)PIPE_META)
                 fail = !mbar_wait_bounded(&bars.done[m], (k / PIPE_META + 1u) & 1u, st.err);
@@ -599,7 +603,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
         const size_t ok_n = out_k.size(), ov_n = out_v.size();
         for (uint32_t k = warp - PIPE_COMPUTE * G;; k += PIPE_STORE) {
             const uint32_t m = k % PIPE_META;
-            if (pipe_store_wait<S>(bars, k, &m_last, st.err)) return;
+            if (pipe_store_wait<S, L>(bars, k, &m_last, st.err)) return;
             const uint32_t cnt = m_cnt[m], start = m_start[m];
             const size_t base = m_base[m];
             const bool enters = m_open[m] && m_carry_h[m];  // the first result's segment began earlier
@@ -642,7 +646,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
         bool aligned = KTMA;
         if constexpr (KTMA) aligned = aligned && (reinterpret_cast<size_t>(keys._data) & 15u) == 0;
         if constexpr (VTMA) aligned = aligned && (reinterpret_cast<size_t>(vals._data) & 15u) == 0;
-        pipe_produce<G, S>(bars, st, tiles, s_first, s_tile, s_bulk, [&](uint32_t s, uint32_t tile, unsigned long long* full) -> bool {
+        pipe_produce<G, S, L>(bars, st, tiles, s_first, s_tile, s_bulk, [&](uint32_t s, uint32_t tile, unsigned long long* full) -> bool {
             const size_t base = (size_t)tile * TILE;
             if (!aligned || base + TILE + HALO > n) return false;
             if constexpr (KTMA) {
@@ -696,7 +700,8 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
     constexpr bool NEIGH = MODE == CM_UNIQUE || MODE == CM_UNIQUE_PRED;
     static_assert(ITEMS < 32 && C >= (int)TILE, "selection mask; a tile's elements fit the ring");
     extern __shared__ __align__(16) unsigned char pipe_smem[];
-    __shared__ PipeBars<S> bars;
+    constexpr int L = S % G == 0 ? S : S * G;
+    __shared__ PipeBars<S, L> bars;
     __shared__ uint32_t s_tile[S], s_bulk[S];
     __shared__ uint32_t m_tile[PIPE_META], m_cnt[PIPE_META], m_all[PIPE_META], m_start[PIPE_META], m_base[PIPE_META];
     __shared__ uint32_t m_end[2 * PIPE_META], m_stored[2 * PIPE_META];  // as in rbk_pipe_kernel
@@ -718,7 +723,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
         constexpr int HALF = PipeShape<G>::WARPS / 2;
         Plus plus;
         if (warp < HALF)
-            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, tiles, plus, reinterpret_cast<unsigned long long*>(st.result), 0u, 1u);
+            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, st, tiles, plus, reinterpret_cast<unsigned long long*>(st.result), 0u, 1u);
         return;
     }
     constexpr uint32_t GT = PIPE_COMPUTE * 32;  // threads of a group
@@ -730,7 +735,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
         uint32_t tail = 0, oldest = 0;
         for (uint32_t k = g;; k += G) {
             const uint32_t s = k % S, m = k % PIPE_META, b = (k / G % 2u) * G + g;
-            bool fail = !mbar_wait_bounded(&bars.full[s], (k / S) & 1u, st.err);
+            bool fail = !mbar_wait_bounded(&bars.full[k % L], (k / L) & 1u, st.err);
             if (!fail && k >= (uint32_t)PIPE_META)
                 fail = !mbar_wait_bounded(&bars.done[m], (k / PIPE_META + 1u) & 1u, st.err);
             if (fail) report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
@@ -830,7 +835,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
         const size_t out_n = out.size();
         for (uint32_t k = warp - PIPE_COMPUTE * G;; k += PIPE_STORE) {
             const uint32_t m = k % PIPE_META;
-            if (pipe_store_wait<S>(bars, k, &m_last, st.err)) return;
+            if (pipe_store_wait<S, L>(bars, k, &m_last, st.err)) return;
             const uint32_t cnt = m_cnt[m], start = m_start[m];
             const size_t base = m_base[m];
             const size_t lim = base >= out_n ? 0 : out_n - base;
@@ -865,12 +870,276 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
     } else if (warp == PIPE_COMPUTE * G + PIPE_STORE + 1 && lane == 0) {
         // ------------------------------------------------------------ producer
         const bool aligned = (reinterpret_cast<size_t>(in) & 15u) == 0;
-        pipe_produce<G, S>(bars, st, tiles, s_first, s_tile, s_bulk, [&](uint32_t s, uint32_t tile, unsigned long long* full) -> bool {
+        pipe_produce<G, S, L>(bars, st, tiles, s_first, s_tile, s_bulk, [&](uint32_t s, uint32_t tile, unsigned long long* full) -> bool {
             const size_t base = (size_t)tile * TILE;
             if (!aligned || base + TILE > n) return false;
             const uint32_t lead = NEIGH && base > 0 ? (uint32_t)SM::LEAD : 0u;
             s_bulk[s] = 1u;
             bulk_load_g2s(stage(s) - (int)lead, in + base - lead, (TILE + lead) * (uint32_t)sizeof(E), full);
+            return true;
+        });
+    }
+}
+
+// ---------------------------------------------------------------- segmented scan
+// Shapes of the segmented scan: 2 groups, tiles of 20 or 10 elements per thread (odd multiples of 16
+// bytes, as above), 3 input stages, and slots for 4 tiles of results.
+template <class K, class T> struct SpipeShape {
+    static constexpr int G = 2, S = 3, R = 4, ITEMS = sizeof(K) + sizeof(T) <= 8 ? 20 : 10;
+    static constexpr int TILE = PIPE_COMPUTE * 32 * ITEMS, HALO = 16 / (int)sizeof(K);
+    static constexpr size_t KEY_BYTES = (size_t)(TILE + HALO) * sizeof(K);
+    static constexpr size_t STAGE = KEY_BYTES + (size_t)TILE * sizeof(T);
+    static constexpr size_t SLOTS = S * STAGE;
+    static constexpr size_t SMEM = SLOTS + (size_t)R * TILE * sizeof(T);
+};
+
+// Scan of the values within segments of equal consecutive keys (EqualTo, Plus; MODE 0 inclusive,
+// MODE 1 exclusive behind init) of contiguous arrays.  The tile is scanned on chip without what
+// enters it; the store warps add that to the elements before its first head.  What enters a tile is
+// the aggregate of the tile before when that holds a head (polled directly), else the prefix CTA's
+// answer.  out may be vals itself; it does not overlap the keys.
+// st: published words, st2: answers.
+template <class K, class T, int MODE>
+__global__ void __launch_bounds__(PipeShape<SpipeShape<K, T>::G>::THREADS, 1) scan_by_key_pipe_kernel(const K* keys, const T* vals, T* out,
+                                                                                                      size_t n, uint32_t tiles, T init,
+                                                                                                      LookbackState st, LookbackState st2) {
+    typedef SpipeShape<K, T> SH;
+    constexpr int G = SH::G, S = SH::S, R = SH::R, ITEMS = SH::ITEMS;
+    constexpr uint32_t TILE = SH::TILE;
+    constexpr uint32_t OWN = (1u << ITEMS) - 1u;
+    constexpr int VEC = 16 / (int)sizeof(T);
+    extern __shared__ __align__(16) unsigned char pipe_smem[];
+    constexpr int L = S % G == 0 ? S : S * G;
+    __shared__ PipeBars<S, L> bars;
+    __shared__ uint32_t s_tile[S], s_bulk[S];
+    __shared__ uint32_t m_tile[PIPE_META], m_first[PIPE_META], m_carry_h[PIPE_META];  // (m_first: the tile's first head)
+    __shared__ T m_carry[PIPE_META];
+    __shared__ T s_wtot[2 * G][PIPE_COMPUTE];
+    __shared__ uint32_t s_wfirst[2 * G][PIPE_COMPUTE];  // the warp's first head, TILE when it holds none
+    __shared__ uint32_t m_last;
+    __shared__ unsigned long long s_first;
+
+    const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
+    auto skey = [&](uint32_t s) -> K* { return reinterpret_cast<K*>(pipe_smem + s * SH::STAGE) + SH::HALO; };
+    auto sval = [&](uint32_t s) -> T* { return reinterpret_cast<T*>(pipe_smem + s * SH::STAGE + SH::KEY_BYTES); };
+    auto slot = [&](uint32_t k) -> T* { return reinterpret_cast<T*>(pipe_smem + SH::SLOTS) + (size_t)(k % R) * TILE; };
+    if (threadIdx.x == 0) {
+        bars.init(1u);
+        m_last = 0xFFFFFFFFu;
+        s_first = atomicAdd(st.tile_ctr, 1ull);
+    }
+    __syncthreads();
+    Plus op;
+    if (s_first == 0) {
+        constexpr int HALF = PipeShape<G>::WARPS / 2;
+        if (warp < HALF) pipe_prefix_scan<T, Plus, true, HALF>(st, st2, tiles, op, nullptr, 0u, 1u);
+        return;
+    }
+    constexpr uint32_t GT = PIPE_COMPUTE * 32;  // threads of a group
+
+    if (warp < PIPE_COMPUTE * G) {
+        // ------------------------------------------------------------ compute
+        const uint32_t g = warp / PIPE_COMPUTE, gw = warp % PIPE_COMPUTE, gt = threadIdx.x % GT, bar = 1u + g;
+        const uint32_t t0 = gt * ITEMS;
+        for (uint32_t k = g;; k += G) {
+            const uint32_t s = k % S, m = k % PIPE_META, b = (k / G % 2u) * G + g;
+            const bool fail = !mbar_wait_bounded(&bars.full[k % L], (k / L) & 1u, st.err);
+            if (fail) report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
+            if (pipe_any(bar, GT, fail)) return;
+            const uint32_t tile = s_tile[s];
+            if (gt == 0) m_tile[m] = tile;  // (free: tile k - R, later than k - PIPE_META, is waited for below)
+            if (tile == PIPE_END) {
+                if (gt == 0) {
+                    atomicMin(&m_last, k);
+                    mbar_arrive(&bars.agg[m]);
+                }
+                return;
+            }
+            const size_t base = (size_t)tile * TILE;
+            const uint32_t cnt = (n - base) < (size_t)TILE ? (uint32_t)(n - base) : TILE;
+            K* kp = skey(s);
+            T* vp = sval(s);
+            if (!s_bulk[s]) {
+                for (uint32_t i = gt; i < cnt; i += GT) {
+                    kp[i] = keys[base + i];
+                    vp[i] = vals[base + i];
+                }
+                if (gt == 0 && base > 0) kp[-1] = keys[base - 1];
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                pipe_sync(bar, GT);
+            }
+            K kk[ITEMS];
+            T x[ITEMS];
+            pipe_load_run<K, ITEMS>(kp + t0, kk);
+            pipe_load_run<T, ITEMS>(vp + t0, x);
+            K prevk = shfl_up_any(kk[ITEMS - 1], 1);
+            if (lane == 0) prevk = kp[(int)t0 - 1];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.empty[s]);
+            uint32_t hd = 0;  // bit j: element j starts a segment
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++)
+                if (!(kk[j] == (j == 0 ? prevk : kk[j > 0 ? j - 1 : 0]))) hd |= 1u << j;
+            if (cnt < TILE) {
+                // elements past the end count as heads of value T(); they are not stored
+                const uint32_t left = cnt > t0 ? cnt - t0 : 0u;
+                if (left < (uint32_t)ITEMS) {
+                    hd |= OWN & ~((1u << left) - 1u);
+#pragma unroll
+                    for (int j = 0; j < ITEMS; j++)
+                        if (j >= (int)left) x[j] = T();
+                }
+            }
+            if (tile == 0 && gt == 0) hd |= 1u;
+            // running values from the lane's first element or the last head on
+#pragma unroll
+            for (int j = 1; j < ITEMS; j++)
+                if (!((hd >> j) & 1u)) x[j] = (T)op(x[j - 1], x[j]);
+            const uint32_t hm = __ballot_sync(0xffffffffu, hd != 0u);
+            const uint32_t le = lane == 31u ? 0xffffffffu : ((2u << lane) - 1u);  // lanes <= l
+            const uint32_t dist = (hm & le) ? lane - (31u - (uint32_t)__clz(hm & le)) : lane;
+            T inc = x[ITEMS - 1];
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const T y = shfl_up_any(inc, d);
+                if ((uint32_t)d <= dist) inc = (T)op(y, inc);
+            }
+            const T ex = shfl_up_any(inc, 1);
+            const bool exhd = (hm & (le >> 1)) != 0u;  // a head in lanes < l
+            if (lane == 31) s_wtot[b][gw] = inc;
+            if (hm == 0u ? lane == 0u : lane == (uint32_t)__ffs(hm) - 1u)
+                s_wfirst[b][gw] = hm == 0u ? TILE : t0 + (uint32_t)__ffs(hd) - 1u;
+            pipe_sync(bar, GT);
+            const uint32_t wf = lane < (uint32_t)PIPE_COMPUTE ? s_wfirst[b][lane] : TILE;
+            const uint32_t wall = __ballot_sync(0xffffffffu, wf != TILE);  // warps holding heads
+            const uint32_t first = __reduce_min_sync(0xffffffffu, wf);
+            const uint32_t whd = wall & ((1u << gw) - 1u);
+            T run = T();
+            bool run_h = gw > 0u;
+            if (gw > 0u) {
+                uint32_t w = whd ? 31u - (uint32_t)__clz(whd) : 0u;
+                run = s_wtot[b][w];
+#pragma unroll 1
+                for (w++; w < gw; w++) run = (T)op(run, s_wtot[b][w]);
+            }
+            if (gw == PIPE_COMPUTE - 1 && lane == 31) {
+                const T agg = (!run_h || hm) ? inc : (T)op(run, inc);
+                pipe_put<T>(st, tile, agg, wall ? 5u : 1u);
+                m_first[m] = first;
+                mbar_arrive(&bars.agg[m]);
+            }
+            if (lane > 0) {
+                run = (exhd || !run_h) ? ex : (T)op(run, ex);
+                run_h = true;
+            }
+            // the lane's elements before its first head continue what precedes the lane in the tile
+            const uint32_t lf = hd ? (uint32_t)__ffs(hd) - 1u : (uint32_t)ITEMS;
+            if (run_h) {
+#pragma unroll
+                for (int j = 0; j < ITEMS; j++)
+                    if (j < (int)lf) x[j] = (T)op(run, x[j]);
+            }
+            if constexpr (MODE == 1) {
+                // the value before each element; before the tile's first head (where what enters the
+                // tile comes in as well) bare, behind it with init in front
+                T before = run;  // (T() at the tile's first element)
+#pragma unroll
+                for (int j = 0; j < ITEMS; j++) {
+                    const T y = x[j];
+                    const bool open = t0 + (uint32_t)j < first;
+                    x[j] = ((hd >> j) & 1u) ? init : open ? before : (T)op(init, before);
+                    before = y;
+                }
+            }
+            // the slot's last tile is written
+            if (k >= (uint32_t)R && !mbar_wait_bounded(&bars.done[(k - R) % PIPE_META], ((k - R) / PIPE_META) & 1u, st.err))
+                report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
+            T* r = slot(k) + t0;
+            if constexpr (ITEMS * sizeof(T) % 16 == 0) {
+                union U { uint4 q[ITEMS * sizeof(T) / 16]; T t[ITEMS]; TRTC_FORCEINLINE U() {} } u;
+#pragma unroll
+                for (int j = 0; j < ITEMS; j++) u.t[j] = x[j];
+#pragma unroll
+                for (int j = 0; j < (int)(ITEMS * sizeof(T) / 16); j++) reinterpret_cast<uint4*>(r)[j] = u.q[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < ITEMS; j++) r[j] = x[j];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.comp[m]);
+        }
+    } else if (warp < PIPE_COMPUTE * G + PIPE_STORE) {
+        // ------------------------------------------------------------ store
+        const bool aligned = (reinterpret_cast<size_t>(out) & 15u) == 0;
+        for (uint32_t k = warp - PIPE_COMPUTE * G;; k += PIPE_STORE) {
+            const uint32_t m = k % PIPE_META;
+            if (pipe_store_wait<S, L>(bars, k, &m_last, st.err)) return;
+            const size_t base = (size_t)m_tile[m] * TILE;
+            const uint32_t cnt = (n - base) < (size_t)TILE ? (uint32_t)(n - base) : TILE;
+            const bool has = m_carry_h[m] != 0u;
+            const uint32_t first = m_first[m] < cnt ? m_first[m] : cnt;
+            const T carry = m_carry[m];
+            // with what enters the tile (i is before the tile's first head)
+            auto entered = [&](uint32_t i, const T& v) -> T {
+                if constexpr (MODE == 0) return has ? (T)op(carry, v) : v;
+                else return (T)op(init, i == 0 ? carry : has ? (T)op(carry, v) : v);
+            };
+            const T* r = slot(k);
+            if (aligned && cnt == TILE) {
+#pragma unroll 4
+                for (uint32_t i = lane * VEC; i < TILE; i += 32 * VEC) {
+                    union { uint4 q; T t[VEC]; } u;
+                    u.q = *reinterpret_cast<const uint4*>(r + i);
+                    if (i < first) {
+#pragma unroll
+                        for (int e = 0; e < VEC; e++)
+                            if (i + e < first) u.t[e] = entered(i + e, u.t[e]);
+                    }
+                    __stcs(reinterpret_cast<uint4*>(out + base + i), u.q);
+                }
+            } else {
+                for (uint32_t i = lane; i < cnt; i += 32) {
+                    T v = r[i];
+                    if (i < first) v = entered(i, v);
+                    out[base + i] = v;
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.done[m]);
+        }
+    } else if (warp == PIPE_COMPUTE * G + PIPE_STORE) {
+        // ------------------------------------------------------------ await
+        pipe_await_slots(bars.agg, bars.pref, m_tile, st.err, [&](uint32_t m, uint32_t tile) -> bool {
+            T v = T();
+            uint32_t f = 0;
+            if (tile > 0) {
+                f = pipe_peek<T>(st, tile - 1u, v);
+                if (f == 5u) {
+                    if constexpr (!LbPack<T>::value) {
+                        fence_acq_rel();
+                        v = reinterpret_cast<const T*>(st.agg)[tile - 1u];
+                    }
+                } else {
+                    f = pipe_answer<T>(st2, tile, v);
+                    if (!f) return false;
+                }
+            }
+            m_carry[m] = v;
+            m_carry_h[m] = (f & 4u) ? 1u : 0u;
+            return true;
+        });
+    } else if (warp == PIPE_COMPUTE * G + PIPE_STORE + 1 && lane == 0) {
+        // ------------------------------------------------------------ producer
+        const bool aligned = ((reinterpret_cast<size_t>(keys) | reinterpret_cast<size_t>(vals)) & 15u) == 0;
+        pipe_produce<G, S, L>(bars, st, tiles, s_first, s_tile, s_bulk, [&](uint32_t s, uint32_t tile, unsigned long long* full) -> bool {
+            const size_t base = (size_t)tile * TILE;
+            if (!aligned || base + TILE > n) return false;
+            const uint32_t lead = base > 0 ? (uint32_t)SH::HALO : 0u;
+            const uint32_t kb = (TILE + lead) * (uint32_t)sizeof(K), vb = TILE * (uint32_t)sizeof(T);
+            s_bulk[s] = 1u;
+            mbar_arrive_expect(full, kb + vb);
+            bulk_load_g2s_more(skey(s) - (int)lead, keys + base - lead, kb, full);
+            bulk_load_g2s_more(sval(s), vals + base, vb, full);
             return true;
         });
     }

@@ -195,6 +195,44 @@ bool reduce_raw(int tc, int op, const void* in, size_t n, const void* init, void
 template <class K, class T, int MODE>
 static bool sbk_t(const K* keys, const T* vals, T* out, size_t n, const T* init, cudaStream_t s) {
     const bool out_over_keys = (const void*)out < (const void*)(keys + n) && (const void*)keys < (const void*)(out + n);
+    const bool apart = (const void*)vals == (const void*)out || (const void*)(vals + n) <= (const void*)out ||
+                       (const void*)(out + n) <= (const void*)vals;
+    const bool aligned = ((reinterpret_cast<size_t>(keys) | reinterpret_cast<size_t>(vals)) & 15u) == 0;
+    // From 48 MiB of aligned keys and values on: the tile pipeline.  B200, us per call, former kernel
+    // against pipeline, int32 keys in runs of 32 with floats: 1 M 8.4 / 12.3, 20 M 67 / 49, 100 M 294 /
+    // 193 (0.96 of the copy rate); int64 keys with floats 20 M 149 / 67, int32 with doubles 227 / 113, int64
+    // with doubles 168 / 121; one segment, 100 M 362 / 268; unaligned 20 M 90 / 94.  Below that size the
+    // pipeline's hand-overs (8 us) are the longer.
+    if (!out_over_keys && apart && aligned && n * (sizeof(K) + sizeof(T)) >= (48ull << 20) && n < 0xFFFFFFFFull) {
+        typedef SpipeShape<K, T> SH;
+        const size_t tiles = (n + SH::TILE - 1) / SH::TILE;
+        uint32_t e8 = 0;
+        LookbackWs* w = lookback_ws(s, tiles, sizeof(T), &e8);
+        if (!w) return false;
+        LookbackState st;
+        st.flags = w->flags;
+        st.agg = w->agg;
+        st.incl = w->incl;
+        st.packed = w->packed;
+        st.tile_ctr = w->tile_ctr;
+        st.epoch8 = e8;
+        st.err = device_error_word();
+        st.result = nullptr;
+        LookbackState st2 = st;  // the answers
+        st2.packed = w->packed2;
+        st2.flags = w->flags2;
+        auto kernel = scan_by_key_pipe_kernel<K, T, MODE>;
+        static const bool ready =
+            TRTC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::SMEM));
+        if (!ready) return false;
+        const size_t g = (size_t)sm_count();  // one of them the prefix CTA
+        ktimer_mark("", s);
+        kernel<<<(unsigned)(g < tiles + 1 ? g : tiles + 1), PipeShape<SH::G>::THREADS, SH::SMEM, s>>>(
+            keys, vals, out, n, (uint32_t)tiles, init ? *init : T(), st, st2);
+        count_launch();
+        ktimer_mark("scan_by_key_kernel", s);
+        return TRTC_CUDA(cudaGetLastError());
+    }
     if constexpr (TRTC_SBK2 && sizeof(K) == sizeof(T) && (sizeof(T) == 4 || sizeof(T) == 8)) {
         if (!out_over_keys) {
             constexpr int ITEMS = TRTC_SBK2_ITEMS * 4 / (int)sizeof(T) < VecWidth<T>::V
@@ -297,7 +335,7 @@ static bool compact_t(const T* in, T* out, size_t n, const T* value, cudaStream_
         (void)cudaGetLastError();  // the failed allocation must not fail the launch check below
     }
     if constexpr ((sizeof(T) == 4 || sizeof(T) == 8) && sizeof(CT) == 4) {
-        if (disjoint) {
+        if (disjoint && n >= COMPACT_PIPE_N) {
             // 4- and 8-byte elements: the tile pipeline (B200, 100 M int32: remove of few 202 -> 195 us
             // per call, unique of runs of 32 157 -> 106, of 2 177 -> 129; int64 unique 339 -> 189)
             typedef CpipeShape<T> SH;

@@ -585,7 +585,7 @@ unsigned long long run_compact(CompactSpec& c) {
                            c.mode == CM_UNIQUE_PRED;
     const size_t es = c.in->elem_size();
     if (two_phase && pipe_mode && !c.two && !c.stencil && (es == 4 || (es == 8 && !c.partition)) && c.in->contiguous_data() &&
-        n < 0xFFFFFFFFull) {
+        n >= COMPACT_PIPE_N && n < 0xFFFFFFFFull) {
         const int items = 80 / (int)es, stages = 3;  // (CpipeShape)
         const size_t tile = (size_t)256 * items, tiles = (n + tile - 1) / tile;
         const size_t stage = tile * es + 16;

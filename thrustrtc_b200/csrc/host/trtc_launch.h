@@ -15,6 +15,12 @@ enum : int { COMPACT_NOT_EQUAL = 2, COMPACT_UNIQUE = 5 };
 // 8: 167 / 51 / 23.4 / 14.4)
 enum : int { REDUCE_CTAS = 4 };
 
+// compactions of fewer elements keep the two-phase kernel, whose one tile per CTA is done before the
+// pipeline has handed a tile through its roles (B200, us per Copy_If / Remove_Copy call, two-phase
+// against pipeline: 5,000 int32 20.3 / 16.9 against 22.2 / 20.9, 1 M 21.0 / 18.0 against 22.7 / 21.3,
+// 4 M 25.8 / 24.7, 10 M 33 / 35 against 30.8 / 32.7)
+enum : unsigned long long { COMPACT_PIPE_N = 1ull << 22 };
+
 // radix sort of built-in key types; vals may be null; vsize = payload bytes per element
 bool sort_raw(int key_tc, void* keys, void* vals, size_t vsize, size_t n, bool desc, cudaStream_t s);
 bool sort_raw_narrow(int key_tc, void* keys, void* vals, size_t vsize, size_t n, bool desc, cudaStream_t s);

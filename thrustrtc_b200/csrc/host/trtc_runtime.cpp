@@ -201,11 +201,11 @@ LookbackWs* lookback_ws(cudaStream_t s, size_t tiles, size_t value_size, uint32_
             if (cap < 1024) cap = 1024;
             size_t vcap = value_size > w->value_cap ? value_size : w->value_cap;
             cudaFree(w->flags); cudaFree(w->agg); cudaFree(w->incl); cudaFree(w->packed);
-            cudaFree(w->packed2);
-            w->flags = nullptr; w->agg = w->incl = nullptr; w->packed = w->packed2 = nullptr;
+            cudaFree(w->packed2); cudaFree(w->flags2);
+            w->flags = w->flags2 = nullptr; w->agg = w->incl = nullptr; w->packed = w->packed2 = nullptr;
             if (!TRTC_CUDA(cudaMalloc(&w->flags, cap * 4)) || !TRTC_CUDA(cudaMalloc(&w->agg, cap * vcap)) ||
                 !TRTC_CUDA(cudaMalloc(&w->incl, cap * vcap)) || !TRTC_CUDA(cudaMalloc(&w->packed, cap * 8)) ||
-                !TRTC_CUDA(cudaMalloc(&w->packed2, cap * 8))) {
+                !TRTC_CUDA(cudaMalloc(&w->packed2, cap * 8)) || !TRTC_CUDA(cudaMalloc(&w->flags2, cap * 4))) {
                 w->tiles_cap = 0;
                 return nullptr;
             }
@@ -218,6 +218,7 @@ LookbackWs* lookback_ws(cudaStream_t s, size_t tiles, size_t value_size, uint32_
         cudaMemset(w->flags, 0, w->tiles_cap * 4);
         cudaMemset(w->packed, 0, w->tiles_cap * 8);
         cudaMemset(w->packed2, 0, w->tiles_cap * 8);
+        cudaMemset(w->flags2, 0, w->tiles_cap * 4);
         cudaMemset(w->tile_ctr, 0, 16);
         cudaDeviceSynchronize();
         w->epoch = 0;

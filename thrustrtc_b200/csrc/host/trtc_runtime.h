@@ -46,7 +46,9 @@ struct LookbackWs {
     void* agg = nullptr;
     void* incl = nullptr;
     unsigned long long* packed = nullptr;  // flag + value words for values of <= 4 bytes
-    unsigned long long* packed2 = nullptr; // a second set, for kernels with two look-backs
+    unsigned long long* packed2 = nullptr; // a second set, for kernels with two streams of words
+    uint32_t* flags2 = nullptr;            // (a word is only ever read as what it was written as: a
+                                           // value's bits could pass for a flag)
     unsigned long long* tile_ctr = nullptr;
     unsigned long long* result = nullptr;  // device scalar (count / total)
     size_t tiles_cap = 0;
