@@ -8,20 +8,24 @@
 // in one of six size classes (ITEMS and warp_small are the tuning table's; launch_segmented.cu):
 //   * segments of at most `warp_small` (0 or 32) keys: one warp, a bitonic network over
 //     (code, index) pairs, no digit counters (seg_warp_bitonic);
-//   * segments of at most 32 * ITEMS keys: one warp, four 8-bit LSD passes of ballot
-//     ranking with per-warp counters (seg_warp_sort_scan); a CTA's eight warps take eight
+//   * segments of at most 32 * ITEMS keys: one warp, 8-bit LSD passes of ballot
+//     ranking (two or three by the top varying bits and a fix-up of ties, SegPlan, else all) with per-warp counters (seg_warp_sort_scan); a CTA's eight warps take eight
 //     such segments at once;
 //   * segments of at most 64 * ITEMS / 128 * ITEMS keys: a group of two / four warps, the
 //     same passes with the group's counters scanned by the group and named barriers of the
 //     group only (seg_group_sort_scan); a CTA's four / two groups take as many segments;
-//   * small segments (<= 256 * ITEMS keys) are sorted on chip: four 8-bit LSD passes of
+//   * small segments (<= 256 * ITEMS keys) are sorted on chip: the same passes of
 //     warp multisplit ranking + shared-memory scatter, with the tile re-laid out so that
 //     every warp gets keys whatever the segment length; then the values are scanned and
 //     keys, values and scan are written once;
-//   * larger segments are sorted by the CTA in global memory: one read builds all digit
-//     histograms, then four chunked, stable scatter passes ping-pong between the segment and
-//     a temp array (mostly L2-resident for segments of up to a few MB), then a chunked
-//     scan with a running carry.
+//   * larger segments: from two tiles up one stable scatter pass through the temp array cuts
+//     the segment into up to 256 buckets by its top varying bits, and the bucket counts carry
+//     the value sums that start each bucket's scan; the CTA's warps, then groups of warps, then
+//     the whole CTA sort and scan the buckets on chip.  Shorter ones, and segments with a
+//     bucket above a tile, take LSD passes in global memory: one read builds all digit
+//     histograms, chunked, stable scatter passes ping-pong between the segment and the temp
+//     array (mostly L2-resident for segments of up to a few MB), then a chunked scan with a
+//     running carry.
 // The queue lists the segments by class, largest first, so the longest work starts first and
 // a CTA's batch of small segments shares one class.
 #pragma once
@@ -76,21 +80,183 @@ __global__ void __launch_bounds__(256) seg_class_count_kernel(const OFF* __restr
     if (threadIdx.x < SEG_CLASSES && s_c[threadIdx.x]) atomicAdd(&ctrl->count[threadIdx.x], s_c[threadIdx.x]);
 }
 
-// queue[] = the segments ordered by class, largest class first (order inside a class is free)
+// queue[] = the segments ordered by class, largest class first (order inside a class is free).
+// A CTA reserves the places of its 256 segments with one atomic per class: one per segment
+// serialised on the few class words (100k segments: 66 us for the count and this kernel, now 21).
 template <class OFF>
 __global__ void __launch_bounds__(256) seg_queue_kernel(const OFF* __restrict__ off, unsigned long long nseg,
                                                         uint32_t items, uint32_t* __restrict__ queue, SegCtrl* ctrl) {
-    __shared__ unsigned long long s_start[SEG_CLASSES];
+    __shared__ unsigned long long s_start[SEG_CLASSES], s_base[SEG_CLASSES];
+    __shared__ uint32_t s_n[SEG_CLASSES];
     if (threadIdx.x == 0) {
         unsigned long long run = 0;
         for (int c = SEG_CLASSES - 1; c >= 0; c--) { s_start[c] = run; run += ctrl->count[c]; }
     }
-    __syncthreads();
-    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < nseg;
-         i += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint32_t c = seg_class((unsigned long long)(off[i + 1] - off[i]), items);
-        queue[s_start[c] + atomicAdd(&ctrl->placed[c], 1ull)] = (uint32_t)i;
+    for (unsigned long long b = (unsigned long long)blockIdx.x * blockDim.x; b < nseg;
+         b += (unsigned long long)gridDim.x * blockDim.x) {
+        if (threadIdx.x < SEG_CLASSES) s_n[threadIdx.x] = 0;
+        __syncthreads();
+        const unsigned long long i = b + threadIdx.x;
+        uint32_t c = 0, r = 0;
+        if (i < nseg) {
+            c = seg_class((unsigned long long)(off[i + 1] - off[i]), items);
+            r = atomicAdd(&s_n[c], 1u);
+        }
+        __syncthreads();
+        if (threadIdx.x < SEG_CLASSES && s_n[threadIdx.x])
+            s_base[threadIdx.x] = s_start[threadIdx.x] + atomicAdd(&ctrl->placed[threadIdx.x], (unsigned long long)s_n[threadIdx.x]);
+        __syncthreads();
+        if (i < nseg) queue[s_base[c] + r] = (uint32_t)i;
+        __syncthreads();
     }
+}
+
+// ------------------------------------------------------------------ which digits a segment needs
+// A segment of n keys is told apart by far fewer bits than its keys have: the top 16 of the
+// bits that vary in it leave n^2 / 2^17 pairs of uniform keys tied (0.5 of a pair at n = 256,
+// 32 at 2048).  So a segment is sorted by those bits only, two 8-bit passes, or by the top 24,
+// three, and the short runs of tied keys that are left are finished in place by the thread at
+// each run's first key (stable: a key only passes larger ones).  Bits above the highest
+// varying one take no pass in either form.
+struct SegPlan {
+    uint32_t shift;   // the passes sort the codes' bits shift .. shift + 8 passes - 1
+    uint32_t passes;
+};
+
+template <class K> constexpr uint32_t seg_min_passes() {
+    return is_same<K, float>::value || is_same<K, double>::value ? 3u : 2u;
+}
+
+// longest run of tied keys finished in place; a longer one that is out of order sends the
+// segment to the passes over all its varying bits (any order the short form leaves keeps equal
+// keys in input order, so they start from there)
+enum { SEG_RUN = 16, SEG_FIXED = 1, SEG_LONG = 2 };
+
+// the key's ordered code, descending order folded in
+template <class K, bool DESC>
+TRTC_FORCEINLINE typename RadixKey<K>::U seg_code(typename RadixKey<K>::B k) {
+    typedef typename RadixKey<K>::U U;
+    const U u = RadixKey<K>::ordered(k);
+    return DESC ? (U)~u : u;
+}
+
+template <class K, bool DESC>
+TRTC_FORCEINLINE uint32_t seg_digit(typename RadixKey<K>::B k, uint32_t shift) {
+    return (uint32_t)(seg_code<K, DESC>(k) >> shift) & 0xFFu;
+}
+
+// OR over the warp
+template <class U>
+TRTC_FORCEINLINE U seg_warp_or(U x) {
+    if constexpr (sizeof(U) == 8) {
+        const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)x);
+        const uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)((unsigned long long)x >> 32));
+        return (U)(((unsigned long long)hi << 32) | lo);
+    } else {
+        return (U)__reduce_or_sync(0xffffffffu, (uint32_t)x);
+    }
+}
+
+// true when two of the warp's sampled codes (`in` lanes) agree above `shift` and differ below:
+// 1 in 130 samples of 32 uniform keys at 16 bits, nearly every one of clustered keys
+template <class U>
+__device__ inline bool seg_sample_ties(U code, bool in, uint32_t shift) {
+    bool tie = false;
+    const uint32_t m = __ballot_sync(0xffffffffu, in);
+    if (in) {
+        const uint32_t peers = __match_any_sync(m, code >> shift);
+        const U first = __shfl_sync(m, code, (int)__ffs(peers) - 1);
+        tie = first != code;
+    }
+    return __any_sync(0xffffffffu, tie);
+}
+
+// all varying bits: `diff` has a bit set where two keys of the segment differ
+template <class U>
+TRTC_FORCEINLINE SegPlan seg_full_plan(U diff) {
+    const uint32_t bits = diff ? 64u - (uint32_t)__clzll((long long)(unsigned long long)diff) : 1u;
+    return {0u, (bits + 7u) / 8u};
+}
+
+// the short form of at least `q0` passes where it saves one, leaves less than one tied key in
+// four for uniform keys and `ties(shift)` does not show clustered ones; else all varying bits.
+// q0 is 2 on chip, 3 in global memory, where a tie costs several round trips (2^24 u32 keys in
+// segments of 10,000: 891 us with two passes, 694 with three, 722 with all four), and 3 for
+// floats: sign, exponent and 7 bits of the mantissa tie most keys of a few hundred (2^24 normal
+// floats in segments of 2000: 754 us with two where the samples allow it, 538 with three).
+// B200, 2^24 keys in equal segments, all digits -> this plan, us: u32 of 64 keys 1384 -> 894,
+// 250 570 -> 363, 500 438 -> 289, 2000 500 -> 412; i64 3659 -> 1263, 1388 -> 529, 1067 -> 397,
+// 1072 -> 573; f32 2054 -> 1789, 757 -> 649, 585 -> 499, 548 -> 538.  What bounds it is the
+// instruction rate of the ranking (eight ballots and an atomic per key and pass).
+template <class U, class TIES>
+__device__ inline SegPlan seg_plan(U diff, uint32_t len, uint32_t q0, TIES ties) {
+    const uint32_t bits = diff ? 64u - (uint32_t)__clzll((long long)(unsigned long long)diff) : 1u;
+    for (uint32_t q = q0; q <= 3; q++)
+        if (8u * q < bits && len <= (1u << (8u * q - 2u)) && !ties(bits - 8u * q)) return {bits - 8u * q, q};
+    return seg_full_plan(diff);
+}
+
+// Element e of a segment that is sorted by its bits from `shift` up: if it is the first of a
+// run of tied keys, insertion-sorts the run's first SEG_RUN keys.  The tied bits of a slot do
+// not change while other threads sort their runs, so the neighbours may be read meanwhile.
+template <class K, class V, bool DESC>
+__device__ inline uint32_t seg_fix_run(volatile typename RadixKey<K>::B* sk, V* sv, uint32_t e, uint32_t len,
+                                       uint32_t shift) {
+    typedef typename RadixKey<K>::B KB;
+    typedef typename RadixKey<K>::U U;
+    if (e + 1 >= len) return 0u;
+    const U pre = seg_code<K, DESC>(sk[e]) >> shift;
+    if ((seg_code<K, DESC>(sk[e + 1]) >> shift) != pre) return 0u;
+    if (e > 0 && (seg_code<K, DESC>(sk[e - 1]) >> shift) == pre) return 0u;
+    for (uint32_t j = e + 1; j < len; j++) {
+        const KB kj = sk[j];
+        const U cj = seg_code<K, DESC>(kj);
+        if ((cj >> shift) != pre) break;
+        if (j - e >= (uint32_t)SEG_RUN) return (uint32_t)SEG_FIXED | (uint32_t)SEG_LONG;
+        uint32_t i = j;
+        if (seg_code<K, DESC>(sk[i - 1]) <= cj) continue;
+        const V vj = sv[j];
+        do {
+            sk[i] = sk[i - 1];
+            sv[i] = sv[i - 1];
+            i--;
+        } while (i > e && seg_code<K, DESC>(sk[i - 1]) > cj);
+        sk[i] = kj;
+        sv[i] = vj;
+    }
+    return (uint32_t)SEG_FIXED;
+}
+
+// seg_fix_run for the elements first, first + stride, ... below end: the ties are collected
+// for 32 of them before the first run is sorted, so the lanes of a warp sort their runs at the
+// same time (row by row nearly every row of 32 has one lane with a run)
+template <class K, class V, bool DESC>
+__device__ inline uint32_t seg_fix_runs(typename RadixKey<K>::B* sk, V* sv, uint32_t first, uint32_t stride,
+                                        uint32_t end, uint32_t len, uint32_t shift) {
+    const uint32_t last = min(end, len - 1u);  // the segment's last key starts no run
+    uint32_t fixed = 0;
+    for (; first < last; first += 32u * stride) {
+        uint32_t mask = 0;
+#pragma unroll 4
+        for (uint32_t r = 0; r < 32u; r++) {
+            const uint32_t e = first + r * stride;
+            if (e >= last) break;
+            const bool tie = ((seg_code<K, DESC>(sk[e]) ^ seg_code<K, DESC>(sk[e + 1])) >> shift) == 0;
+            mask |= tie ? 1u << r : 0u;
+        }
+        while (mask) {
+            const uint32_t e = first + (uint32_t)(__ffs((int)mask) - 1) * stride;
+            mask &= mask - 1u;
+            fixed |= seg_fix_run<K, V, DESC>(sk, sv, e, len, shift);
+        }
+    }
+    return fixed;
+}
+
+// true where element e is smaller than the one before it
+template <class K, bool DESC>
+TRTC_FORCEINLINE bool seg_inverted(const volatile typename RadixKey<K>::B* sk, uint32_t e) {
+    return e > 0 && seg_code<K, DESC>(sk[e - 1]) > seg_code<K, DESC>(sk[e]);
 }
 
 // Ranks IT (<= ITEMS) warp-striped items per thread of a tile of `tile_n` keys: element
@@ -98,7 +264,7 @@ __global__ void __launch_bounds__(256) seg_queue_kernel(const OFF* __restrict__ 
 // tile (stable), s_cnt[d] / s_start[d] the tile's digit counts and exclusive starts.
 template <class K, bool DESC, int ITEMS>
 __device__ inline void seg_rank_tile(const typename RadixKey<K>::B (&keys)[ITEMS], uint32_t (&pos)[ITEMS], int IT,
-                                     uint32_t tile_n, uint32_t sel, bool hi, uint32_t* s_whist, uint32_t* s_cnt,
+                                     uint32_t tile_n, uint32_t shift, uint32_t* s_whist, uint32_t* s_cnt,
                                      uint32_t* s_start, uint32_t* s_wsum) {
     constexpr int WARPS = 8;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -114,7 +280,7 @@ __device__ inline void seg_rank_tile(const typename RadixKey<K>::B (&keys)[ITEMS
         info[i] = 0;
         if (i >= IT || wbase + (uint32_t)i * 32u >= tile_n) continue;  // warp-uniform
         const bool valid = wbase + (uint32_t)i * 32u + lane < tile_n;
-        const uint32_t d = radix_digit_sel<K, DESC>(keys[i], sel, hi);
+        const uint32_t d = seg_digit<K, DESC>(keys[i], shift);
         uint32_t peers = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
         for (int b = 0; b < 8; b++) {
@@ -150,7 +316,7 @@ __device__ inline void seg_rank_tile(const typename RadixKey<K>::B (&keys)[ITEMS
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
         if (i >= IT || wbase + (uint32_t)i * 32u + lane >= tile_n) continue;
-        pos[i] += wh[radix_digit_sel<K, DESC>(keys[i], sel, hi)];
+        pos[i] += wh[seg_digit<K, DESC>(keys[i], shift)];
     }
 }
 
@@ -187,12 +353,15 @@ __device__ inline V seg_block_excl_scan(const V* s_v, V* s_o, uint32_t len, V ca
 // One warp sorts (stable LSD, 8-bit digits) and scans a segment of len <= 32 * ITEMS keys on
 // its own: no block barrier, so the CTA's eight warps work on eight small segments at once.
 // Element e = i*32 + lane sits in item i of the lane; sk / sv are this warp's staging slices
-// (32 * ITEMS elements), wh its 256 digit counters.
+// (32 * ITEMS elements), wh its 256 digit counters.  ik / iv: where the keys and values are read
+// (gk / gv for a segment in place); carry: the scan's first value.
 template <class K, class V, bool DESC, int ITEMS>
-__device__ inline void seg_warp_sort_scan(typename RadixKey<K>::B* gk, V* gv, V* gs, uint32_t len,
-                                          typename RadixKey<K>::B* sk, V* sv, uint32_t* wh) {
+__device__ inline void seg_warp_sort_scan(const typename RadixKey<K>::B* ik, const V* iv, typename RadixKey<K>::B* gk,
+                                          V* gv, V* gs, uint32_t len, V carry, typename RadixKey<K>::B* sk, V* sv,
+                                          uint32_t* wh) {
     typedef typename RadixKey<K>::B KB;
-    constexpr int D = RadixKey<K>::DIGITS;
+    typedef typename RadixKey<K>::U U;
+    constexpr uint32_t Q0 = seg_min_passes<K>();
     const uint32_t lane = threadIdx.x & 31u;
     const int IT = (int)((len + 31u) / 32u);  // items in use (warp-uniform)
     const uint32_t ltm = lanemask_lt();
@@ -201,12 +370,20 @@ __device__ inline void seg_warp_sort_scan(typename RadixKey<K>::B* gk, V* gv, V*
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
         const uint32_t e = (uint32_t)i * 32u + lane;
-        if (i < IT && e < len) { k[i] = gk[e]; v[i] = gv[e]; }
+        if (i < IT && e < len) { k[i] = ik[e]; v[i] = iv[e]; }
         else { k[i] = KB(0); v[i] = V(); }
     }
-    for (int p = 0; p < D; p++) {
-        const uint32_t sel = 0x4440u | (uint32_t)(p & 3);
-        const bool hi = p >= 4;
+    const U ref = seg_code<K, DESC>(ik[0]);
+    U diff = 0;
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++)
+        if (i < IT && (uint32_t)i * 32u + lane < len) diff |= seg_code<K, DESC>(k[i]) ^ ref;
+    diff = seg_warp_or(diff);
+    SegPlan plan = seg_plan(diff, len, Q0, [&](uint32_t sh) {
+        return seg_sample_ties(seg_code<K, DESC>(k[0]), lane < len, sh);
+    });
+    uint32_t shift = plan.shift;
+    for (uint32_t p = 0; p < plan.passes; p++) {
 #pragma unroll
         for (int j = 0; j < 8; j++) wh[j * 32 + lane] = 0;
         __syncwarp();
@@ -217,7 +394,7 @@ __device__ inline void seg_warp_sort_scan(typename RadixKey<K>::B* gk, V* gv, V*
             info[i] = 0;
             if (i >= IT) continue;
             const bool valid = (uint32_t)i * 32u + lane < len;
-            const uint32_t d = radix_digit_sel<K, DESC>(k[i], sel, hi);
+            const uint32_t d = seg_digit<K, DESC>(k[i], shift);
             uint32_t peers = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
             for (int b = 0; b < 8; b++) {
@@ -250,7 +427,7 @@ __device__ inline void seg_warp_sort_scan(typename RadixKey<K>::B* gk, V* gv, V*
 #pragma unroll
         for (int i = 0; i < ITEMS; i++) {
             if (i >= IT || (uint32_t)i * 32u + lane >= len) continue;
-            const uint32_t q = pos[i] + wh[radix_digit_sel<K, DESC>(k[i], sel, hi)];
+            const uint32_t q = pos[i] + wh[seg_digit<K, DESC>(k[i], shift)];
             sk[q] = k[i];
             sv[q] = v[i];
         }
@@ -261,9 +438,31 @@ __device__ inline void seg_warp_sort_scan(typename RadixKey<K>::B* gk, V* gv, V*
             if (i < IT && e < len) { k[i] = sk[e]; v[i] = sv[e]; }
         }
         __syncwarp();
+        shift += 8u;
+        if (p + 1 < plan.passes || plan.shift == 0) continue;
+        // the last pass of the short form: the runs of tied keys
+        const uint32_t fixed =
+            __reduce_or_sync(0xffffffffu, seg_fix_runs<K, V, DESC>(sk, sv, lane, 32u, len, len, plan.shift));
+        __syncwarp();
+        if (fixed) {
+#pragma unroll
+            for (int i = 0; i < ITEMS; i++) {
+                const uint32_t e = (uint32_t)i * 32u + lane;
+                if (i < IT && e < len) { k[i] = sk[e]; v[i] = sv[e]; }
+            }
+        }
+        if (fixed & (uint32_t)SEG_LONG) {
+            bool inv = false;
+            for (uint32_t e = lane; e < len; e += 32u) inv |= seg_inverted<K, DESC>(sk, e);
+            if (__any_sync(0xffffffffu, inv)) {
+                plan = seg_full_plan(diff);
+                shift = 0;
+                p = ~0u;  // from the first pass again
+            }
+        }
+        __syncwarp();
     }
     // exclusive scan of the sorted values, written with the sorted keys and values
-    V carry = V();
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
         if (i >= IT) continue;
@@ -296,13 +495,15 @@ __device__ inline void seg_warp_sort_scan(typename RadixKey<K>::B* gk, V* gv, V*
 // meet at its named barrier `bar` (1 + group index, 32 * G threads), so the CTA's 8 / G
 // groups work on 8 / G segments at once.  s_wsum / s_vpart: one slot per warp of the CTA.
 template <class K, class V, bool DESC, int ITEMS>
-__device__ inline void seg_group_sort_scan(typename RadixKey<K>::B* gk, V* gv, V* gs, uint32_t len,
-                                           typename RadixKey<K>::B* sk, V* va, V* vb, uint32_t* s_whist,
-                                           uint32_t* s_wsum, V* s_vpart, uint32_t G, uint32_t bar) {
+__device__ __noinline__ void seg_group_sort_scan(const typename RadixKey<K>::B* ik, const V* iv,
+                                                 typename RadixKey<K>::B* gk, V* gv, V* gs, uint32_t len, V carry,
+                                                 typename RadixKey<K>::B* sk, V* va, V* vb, uint32_t* s_whist,
+                                                 uint32_t* s_wsum, V* s_vpart, uint32_t G, uint32_t bar) {
     // G is a runtime value (2 or 4): one copy of this code serves both group sizes, which
     // keeps the kernel inside its register budget
     typedef typename RadixKey<K>::B KB;
-    constexpr int D = RadixKey<K>::DIGITS;
+    typedef typename RadixKey<K>::U U;
+    constexpr uint32_t Q0 = seg_min_passes<K>();
     const uint32_t GT = 32u * G;      // threads of the group
     const uint32_t DPT = 256u / GT;   // digits scanned per thread
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -326,12 +527,34 @@ __device__ inline void seg_group_sort_scan(typename RadixKey<K>::B* gk, V* gv, V
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
         const uint32_t r = (uint32_t)i * 32u + lane;
-        if ((uint32_t)i < IT && r < wn) { k[i] = gk[wbase + r]; va[wbase + r] = gv[wbase + r]; }
+        if ((uint32_t)i < IT && r < wn) { k[i] = ik[wbase + r]; va[wbase + r] = iv[wbase + r]; }
         else k[i] = KB(0);
     }
-    for (int p = 0; p < D; p++) {
-        const uint32_t sel = 0x4440u | (uint32_t)(p & 3);
-        const bool hi = p >= 4;
+    const U ref = seg_code<K, DESC>(ik[0]);
+    U diff = 0;
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++)
+        if ((uint32_t)i < IT && (uint32_t)i * 32u + lane < wn) diff |= seg_code<K, DESC>(k[i]) ^ ref;
+    diff = seg_warp_or(diff);
+    if (lane == 0) {
+        wh[0] = (uint32_t)diff;
+        wh[1] = (uint32_t)((unsigned long long)diff >> 32);
+    }
+    gsync();
+    for (uint32_t w = 0; w < G; w++) {
+        const uint32_t* cw = &s_whist[(gw0 + w) * 256];
+        diff |= (U)(((unsigned long long)cw[1] << 32) | cw[0]);
+    }
+    // (every warp looks at the same G samples, spread over the segment)
+    SegPlan plan = seg_plan(diff, len, Q0, [&](uint32_t sh) {
+        bool tie = false;
+        for (uint32_t w = 0; w < G; w++)
+            tie |= seg_sample_ties(seg_code<K, DESC>(ik[(len / GT) * (w * 32u + lane)]), true, sh);
+        return tie;
+    });
+    gsync();  // the counters are free
+    uint32_t shift = plan.shift;
+    for (uint32_t p = 0; p < plan.passes; p++) {
 #pragma unroll
         for (int j = 0; j < 8; j++) wh[j * 32 + lane] = 0;
         __syncwarp();
@@ -341,7 +564,7 @@ __device__ inline void seg_group_sort_scan(typename RadixKey<K>::B* gk, V* gv, V
             pos[i] = 0;
             if ((uint32_t)i >= IT || (uint32_t)i * 32u >= wn) continue;  // warp-uniform
             const bool valid = (uint32_t)i * 32u + lane < wn;
-            const uint32_t d = radix_digit_sel<K, DESC>(k[i], sel, hi);
+            const uint32_t d = seg_digit<K, DESC>(k[i], shift);
             uint32_t peers = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
             for (int b = 0; b < 8; b++) {
@@ -382,19 +605,41 @@ __device__ inline void seg_group_sort_scan(typename RadixKey<K>::B* gk, V* gv, V
         for (int i = 0; i < ITEMS; i++) {
             const uint32_t r = (uint32_t)i * 32u + lane;
             if ((uint32_t)i >= IT || r >= wn) continue;
-            const uint32_t q = pos[i] + wh[radix_digit_sel<K, DESC>(k[i], sel, hi)];
+            const uint32_t q = pos[i] + wh[seg_digit<K, DESC>(k[i], shift)];
             sk[q] = k[i];
             vb[q] = va[wbase + r];
         }
         gsync();  // the pass's order is complete in sk / vb
-        if (p + 1 < D) {
-#pragma unroll
-            for (int i = 0; i < ITEMS; i++) {
-                const uint32_t r = (uint32_t)i * 32u + lane;
-                if ((uint32_t)i < IT && r < wn) k[i] = sk[wbase + r];
-            }
-        }
         V* t = va; va = vb; vb = t;
+        shift += 8u;
+        if (p + 1 == plan.passes) {
+            if (plan.shift == 0) break;
+            // the last pass of the short form: the runs of tied keys
+            uint32_t fixed = __reduce_or_sync(
+                0xffffffffu, seg_fix_runs<K, V, DESC>(sk, va, wbase + lane, 32u, wbase + wn, len, plan.shift));
+            if (lane == 0) s_wsum[warp] = fixed;
+            gsync();  // the runs are sorted
+            fixed = 0;
+            for (uint32_t w = 0; w < G; w++) fixed |= s_wsum[gw0 + w];
+            if (!(fixed & (uint32_t)SEG_LONG)) break;
+            bool inv = false;
+            for (uint32_t r = lane; r < wn; r += 32u) inv |= seg_inverted<K, DESC>(sk, wbase + r);
+            inv = __any_sync(0xffffffffu, inv);
+            if (lane == 0) wh[0] = inv ? 1u : 0u;
+            gsync();
+            uint32_t any = 0;
+            for (uint32_t w = 0; w < G; w++) any |= s_whist[(gw0 + w) * 256];
+            gsync();  // the counters are free
+            if (!any) break;
+            plan = seg_full_plan(diff);
+            shift = 0;
+            p = ~0u;  // from the first pass again
+        }
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const uint32_t r = (uint32_t)i * 32u + lane;
+            if ((uint32_t)i < IT && r < wn) k[i] = sk[wbase + r];
+        }
         // the next pass writes sk / vb only after its first group barrier, which every warp
         // reaches after this reload
     }
@@ -408,7 +653,6 @@ __device__ inline void seg_group_sort_scan(typename RadixKey<K>::B* gk, V* gv, V
     for (int d = 16; d > 0; d >>= 1) wsum += shfl_xor_any(wsum, d);
     if (lane == 0) s_vpart[warp] = wsum;
     gsync();
-    V carry = V();
     for (uint32_t w = 0; w < wg; w++) carry += s_vpart[gw0 + w];
 #pragma unroll 1
     for (uint32_t r0 = 0; r0 < wn; r0 += 32u) {  // rows of the warp's chunk (warp-uniform)
@@ -523,6 +767,9 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
     __shared__ V s_part[8];
     __shared__ unsigned long long s_item;
     __shared__ unsigned long long s_batch, s_defer[8];
+    __shared__ uint32_t s_bucket;
+    static_assert(sizeof(typename RadixKey<K>::B) >= 4 && is_same<V, uint32_t>::value,
+                  "keys of 4 or 8 bytes, uint32_t values");
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     constexpr uint32_t WSEG = 32u * ITEMS;  // segments up to this length are sorted by one warp
 
@@ -547,94 +794,59 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
 
     // whole-CTA sort + scan of one segment (on chip up to TILE keys, else through global memory)
     auto block_segment = [&](KB* gk, V* gv, V* gs, uint32_t len, unsigned long long base) {
-        if (len <= (uint32_t)TILE) {
-            // ---------------- on-chip sort of a small segment
-            const int IT = (int)((len + 255u) / 256u);
-            const uint32_t wbase = warp * 32u * (uint32_t)IT;
-            KB k[ITEMS];
-            V v[ITEMS];
-            uint32_t pos[ITEMS];
-#pragma unroll
-            for (int i = 0; i < ITEMS; i++) {
-                const uint32_t e = wbase + (uint32_t)i * 32u + lane;
-                if (i < IT && e < len) { k[i] = gk[e]; v[i] = gv[e]; }
-                else { k[i] = KB(0); v[i] = V(); }
-            }
-            for (int p = 0; p < D; p++) {
-                const uint32_t sel = 0x4440u | (uint32_t)(p & 3);
-                seg_rank_tile<K, DESC, ITEMS>(k, pos, IT, len, sel, p >= 4, s_whist, s_cnt, s_start, s_wsum);
-#pragma unroll
-                for (int i = 0; i < ITEMS; i++) {
-                    const uint32_t e = wbase + (uint32_t)i * 32u + lane;
-                    if (i < IT && e < len) { s_k[pos[i]] = k[i]; s_v[pos[i]] = v[i]; }
-                }
-                __syncthreads();
-                if (p + 1 < D) {
-#pragma unroll
-                    for (int i = 0; i < ITEMS; i++) {
-                        const uint32_t e = wbase + (uint32_t)i * 32u + lane;
-                        if (i < IT && e < len) { k[i] = s_k[e]; v[i] = s_v[e]; }
-                    }
-                }
-                __syncthreads();
-            }
-            // s_k / s_v hold the sorted segment; exclusive scan of the values into s_o
-            if (gs) seg_block_excl_scan<V, ITEMS>(s_v, s_o, len, V(), s_part);
-            for (uint32_t e = threadIdx.x; e < len; e += 256) {
-                gk[e] = s_k[e];
-                gv[e] = s_v[e];
-                if (gs) gs[e] = s_o[e];
-            }
-            return;
-        }
-
-        // ---------------- large segment: CTA-level LSD passes through global memory
-        for (int i = threadIdx.x; i < D * 256; i += 256) (&s_hist[0][0])[i] = 0;
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < len; e += 256) {
-            typename RadixKey<K>::U u = RadixKey<K>::ordered(gk[e]);
-            if (DESC) u = ~u;
-#pragma unroll
-            for (int p = 0; p < D; p++) {
-                const uint32_t w = (p < 4) ? (uint32_t)u : (uint32_t)((unsigned long long)u >> 32);
-                atomicAdd(&s_hist[p][__byte_perm(w, 0u, 0x4440u | (uint32_t)(p & 3))], 1u);
-            }
-        }
-        __syncthreads();
-        KB* sk = gk;
-        V* sv = gv;
-        KB* dk = tk + base;
-        V* dv = tv + base;
-        for (int p = 0; p < D; p++) {
-            const uint32_t sel = 0x4440u | (uint32_t)(p & 3);
-            const bool hi = p >= 4;
-            {
-                const uint32_t c = s_hist[p][threadIdx.x];
-                s_run[threadIdx.x] = block_excl_scan_256<256>(c, s_wsum);
+        typedef typename RadixKey<K>::U U;
+        // OR over the CTA (in the digit counters, which every pass clears first)
+        auto block_or = [&](U x) -> U {
+            x = seg_warp_or(x);
+            __syncthreads();
+            if (lane == 0) {
+                s_whist[2 * warp] = (uint32_t)x;
+                s_whist[2 * warp + 1] = (uint32_t)((unsigned long long)x >> 32);
             }
             __syncthreads();
+            for (int w = 0; w < 8; w++)
+                x |= (U)(((unsigned long long)s_whist[2 * w + 1] << 32) | s_whist[2 * w]);
+            __syncthreads();
+            return x;
+        };
+        // eight samples spread over n >= 256 keys; two ties among uniform keys are 1 in 600
+        auto sampled = [&](const KB* k, uint32_t n, uint32_t sh) -> bool {
+            const bool tie = seg_sample_ties(seg_code<K, DESC>(k[(n >> 8) * threadIdx.x]), true, sh);
+            return __syncthreads_count(tie && lane == 0) >= 2;
+        };
+        // finishes the runs of tied keys that a short form left; false: some run is too long
+        auto sorted_runs = [&](KB* k, V* v, uint32_t n, uint32_t shift) -> bool {
+            const uint32_t fixed = seg_fix_runs<K, V, DESC>(k, v, threadIdx.x, 256u, n, n, shift);
+            if (!__syncthreads_or((int)(fixed & (uint32_t)SEG_LONG))) return true;
+            bool inv = false;
+            for (uint32_t e = threadIdx.x; e < n; e += 256) inv |= seg_inverted<K, DESC>(k, e);
+            return !__syncthreads_or(inv);
+        };
+        // one stable pass by the digit at `shift` through global memory; s_run: the digits' starts
+        auto scatter = [&](const KB* sk, const V* sv, KB* dk, V* dv, uint32_t shift) {
             for (uint32_t cb = 0; cb < len; cb += TILE) {
                 const uint32_t cn = min((uint32_t)TILE, len - cb);
-                const uint32_t wbase = warp * 32u * ITEMS;
+                const int IT = (int)((cn + 255u) / 256u);
+                const uint32_t wbase = warp * 32u * (uint32_t)IT;
                 KB k[ITEMS];
                 V v[ITEMS];
                 uint32_t pos[ITEMS];
 #pragma unroll
                 for (int i = 0; i < ITEMS; i++) {
                     const uint32_t e = wbase + (uint32_t)i * 32u + lane;
-                    if (e < cn) { k[i] = sk[cb + e]; v[i] = sv[cb + e]; }
+                    if (i < IT && e < cn) { k[i] = sk[cb + e]; v[i] = sv[cb + e]; }
                     else { k[i] = KB(0); v[i] = V(); }
                 }
-                seg_rank_tile<K, DESC, ITEMS>(k, pos, ITEMS, cn, sel, hi, s_whist, s_cnt, s_start, s_wsum);
+                seg_rank_tile<K, DESC, ITEMS>(k, pos, IT, cn, shift, s_whist, s_cnt, s_start, s_wsum);
 #pragma unroll
                 for (int i = 0; i < ITEMS; i++) {
                     const uint32_t e = wbase + (uint32_t)i * 32u + lane;
-                    if (e < cn) { s_k[pos[i]] = k[i]; s_v[pos[i]] = v[i]; }
+                    if (i < IT && e < cn) { s_k[pos[i]] = k[i]; s_v[pos[i]] = v[i]; }
                 }
                 __syncthreads();
                 for (uint32_t e = threadIdx.x; e < cn; e += 256) {
                     const KB key = s_k[e];
-                    const uint32_t d = radix_digit_sel<K, DESC>(key, sel, hi);
+                    const uint32_t d = seg_digit<K, DESC>(key, shift);
                     const uint32_t dst = s_run[d] + (e - s_start[d]);
                     dk[dst] = key;
                     dv[dst] = s_v[e];
@@ -643,24 +855,218 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
                 s_run[threadIdx.x] += s_cnt[threadIdx.x];
                 __syncthreads();
             }
-            KB* t1 = sk; sk = dk; dk = t1;
-            V* t2 = sv; sv = dv; dv = t2;
+        };
+        const KB* ck = gk;  // what the on-chip part reads: the segment, or its buckets in tk / tv
+        const V* cv = gv;
+        const bool split = len > (uint32_t)TILE;
+        if (split) {
+            // ---------------- large segment
+            KB* dk = tk + base;
+            V* dv = tv + base;
+            const U ref = seg_code<K, DESC>(gk[0]);
+            // from two CTA tiles up (16 keys a thread: 8192 keys; 2^24 u32 keys in segments of
+            // 40,000: 829 us by LSD passes, 598 this way, one segment of 100,000 951 and 667; one of
+            // 5000 79 and 96):
+            // one pass by the top bits of those that vary puts the keys into buckets of 5/8 of a
+            // warp's share on average (up to 256 of them); each is then sorted on chip.  Which bits
+            // vary is read off a sample of 256 keys and checked by the pass that counts them all.
+            const KB sample = gk[(len >> 8) * threadIdx.x];
+            U diff = block_or(seg_code<K, DESC>(sample) ^ ref);
+            const uint32_t bits = diff ? 64u - (uint32_t)__clzll((long long)(unsigned long long)diff) : 1u;
+            const uint32_t nb = min(8u, 32u - (uint32_t)__clz((len - 1u) / (WSEG * 5u / 8u)));
+            const uint32_t top = bits > nb ? bits - nb : 0u;
+            s_hist[0][threadIdx.x] = 0;
+            s_hist[1][threadIdx.x] = 0;
+            __syncthreads();
+            atomicAdd(&s_hist[0][seg_digit<K, DESC>(sample, top)], 1u);
+            __syncthreads();
+            // (clustered keys, the exponents of floats, fill a bucket: seen in the sample already)
+            const uint32_t seen = s_hist[0][threadIdx.x];
+            bool one = __syncthreads_or(len <= 2u * (uint32_t)TILE ||
+                                        (seen >= 16u && (unsigned long long)seen * (len >> 8) > 2ull * TILE));
+            if (!one) {
+                s_hist[0][threadIdx.x] = 0;
+                __syncthreads();
+                U all = 0;
+                for (uint32_t e = threadIdx.x; e < len; e += 1024) {
+                    KB k[4];
+                    V v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const uint32_t x = min(e + 256u * j, len - 1u);
+                        k[j] = gk[x];
+                        v[j] = gv[x];
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        all |= seg_code<K, DESC>(k[j]) ^ ref;
+                        if (e + 256u * j >= len) continue;
+                        const uint32_t d = seg_digit<K, DESC>(k[j], top);
+                        atomicAdd(&s_hist[0][d], 1u);
+                        atomicAdd(&s_hist[1][d], (uint32_t)v[j]);
+                    }
+                }
+                __syncthreads();
+                const uint32_t c = s_hist[0][threadIdx.x], sum = s_hist[1][threadIdx.x];
+                one = __syncthreads_or(c > (uint32_t)TILE || (all >> top) > U(0xFF));
+                if (!one) {
+                    const uint32_t st = block_excl_scan_256<256>(c, s_wsum);
+                    __syncthreads();
+                    s_hist[2][threadIdx.x] = block_excl_scan_256<256>(sum, s_wsum);  // the scan's value at the bucket
+                    s_hist[1][threadIdx.x] = st;
+                    s_run[threadIdx.x] = st;
+                    __syncthreads();
+                    scatter(gk, gv, dk, dv, top);
+                    if (threadIdx.x == 0) s_bucket = 0;
+                    __syncthreads();
+                    // buckets of up to a warp's share: one warp each
+                    while (true) {
+                        uint32_t b = 0;
+                        if (lane == 0) b = atomicAdd(&s_bucket, 1u);
+                        b = __shfl_sync(0xffffffffu, b, 0);
+                        if (b >= 256u) break;
+                        const uint32_t n = s_hist[0][b], o = s_hist[1][b];
+                        if (n == 0 || n > WSEG) continue;
+                        seg_warp_sort_scan<K, V, DESC, ITEMS>(dk + o, dv + o, gk + o, gv + o, gs ? gs + o : nullptr, n,
+                                                              (V)s_hist[2][b], s_k + warp * WSEG, s_v + warp * WSEG,
+                                                              s_whist + warp * 256);
+                    }
+                    __syncthreads();
+                    // up to two and four shares: groups of two and four warps
+                    for (uint32_t G = 2; G <= 4; G *= 2) {
+                        const uint32_t grp = warp / G;
+                        for (uint32_t b = grp; b < 256u; b += 8u / G) {
+                            const uint32_t n = s_hist[0][b], o = s_hist[1][b];
+                            if (n <= G / 2 * WSEG || n > G * WSEG) continue;
+                            seg_group_sort_scan<K, V, DESC, ITEMS>(
+                                dk + o, dv + o, gk + o, gv + o, gs ? gs + o : nullptr, n, (V)s_hist[2][b],
+                                s_k + grp * G * WSEG, s_v + grp * G * WSEG, s_o + grp * G * WSEG, s_whist, s_wsum,
+                                s_part, G, 1u + grp);
+                        }
+                        __syncthreads();
+                    }
+                    ck = dk;
+                    cv = dv;
+                }
+            }
+            if (one) {
+                // CTA-level LSD passes through global memory
+                KB* sk = gk;
+                V* sv = gv;
+                SegPlan plan;
+                if constexpr (sizeof(U) == 8) {
+                    diff = 0;
+#pragma unroll 4
+                    for (uint32_t e = threadIdx.x; e < len; e += 256) diff |= seg_code<K, DESC>(gk[e]) ^ ref;
+                    diff = block_or(diff);
+                    plan = seg_plan(diff, len, 3u, [&](uint32_t sh) { return sampled(gk, len, sh); });
+                } else {  // (finding the varying bits, three passes and the ties cost as much as four passes)
+                    diff = ~U(0);
+                    plan = seg_full_plan(diff);
+                }
+                while (true) {
+                    for (uint32_t i = threadIdx.x; i < plan.passes * 256u; i += 256u) (&s_hist[0][0])[i] = 0;
+                    __syncthreads();
+                    for (uint32_t e = threadIdx.x; e < len; e += 256) {
+                        const U u = seg_code<K, DESC>(sk[e]) >> plan.shift;
+#pragma unroll
+                        for (int p = 0; p < D; p++) {
+                            if ((uint32_t)p >= plan.passes) break;
+                            const uint32_t w = (p < 4) ? (uint32_t)u : (uint32_t)((unsigned long long)u >> 32);
+                            atomicAdd(&s_hist[p][__byte_perm(w, 0u, 0x4440u | (uint32_t)(p & 3))], 1u);
+                        }
+                    }
+                    __syncthreads();
+                    for (uint32_t p = 0; p < plan.passes; p++) {
+                        const uint32_t shift = plan.shift + 8u * p;
+                        {
+                            const uint32_t c = s_hist[p][threadIdx.x];
+                            s_run[threadIdx.x] = block_excl_scan_256<256>(c, s_wsum);
+                        }
+                        __syncthreads();
+                        scatter(sk, sv, dk, dv, shift);
+                        KB* t1 = sk; sk = dk; dk = t1;
+                        V* t2 = sv; sv = dv; dv = t2;
+                    }
+                    if (plan.shift == 0 || sorted_runs(sk, sv, len, plan.shift)) break;
+                    plan = seg_full_plan(diff);
+                }
+                // the sorted segment is in sk/sv (the caller's arrays after an even number of passes);
+                // chunked exclusive scan with a running carry, writing keys and values back if needed
+                V carry = V();
+                for (uint32_t cb = 0; cb < len; cb += TILE) {
+                    const uint32_t cn = min((uint32_t)TILE, len - cb);
+                    for (uint32_t e = threadIdx.x; e < cn; e += 256) {
+                        s_v[e] = sv[cb + e];
+                        if (sk != gk) { gk[cb + e] = sk[cb + e]; gv[cb + e] = s_v[e]; }
+                    }
+                    __syncthreads();
+                    if (gs) {
+                        carry = seg_block_excl_scan<V, ITEMS>(s_v, s_o, cn, carry, s_part);
+                        for (uint32_t e = threadIdx.x; e < cn; e += 256) gs[cb + e] = s_o[e];
+                    }
+                    __syncthreads();
+                }
+                return;
+            }
         }
-        // after D passes the segment is in sk/sv (the caller's arrays when D is even);
-        // chunked exclusive scan with a running carry, writing keys and values back if needed
-        V carry = V();
-        for (uint32_t cb = 0; cb < len; cb += TILE) {
-            const uint32_t cn = min((uint32_t)TILE, len - cb);
-            for (uint32_t e = threadIdx.x; e < cn; e += 256) {
-                s_v[e] = sv[cb + e];
-                if (sk != gk) { gk[cb + e] = sk[cb + e]; gv[cb + e] = s_v[e]; }
+
+        // ---------------- on-chip sort: the segment, or the buckets above four shares
+        for (uint32_t b = 0; b < (split ? 256u : 1u); b++) {
+            const uint32_t n = split ? s_hist[0][b] : len, st = split ? s_hist[1][b] : 0u;
+            if (split && n <= 4u * WSEG) continue;
+            const V first = split ? (V)s_hist[2][b] : V();
+            const KB* ik = ck + st;
+            const V* iv = cv + st;
+            const int IT = (int)((n + 255u) / 256u);
+            const uint32_t wbase = warp * 32u * (uint32_t)IT;
+            KB k[ITEMS];
+            V v[ITEMS];
+            uint32_t pos[ITEMS];
+#pragma unroll
+            for (int i = 0; i < ITEMS; i++) {
+                const uint32_t e = wbase + (uint32_t)i * 32u + lane;
+                if (i < IT && e < n) { k[i] = ik[e]; v[i] = iv[e]; }
+                else { k[i] = KB(0); v[i] = V(); }
             }
-            __syncthreads();
-            if (gs) {
-                carry = seg_block_excl_scan<V, ITEMS>(s_v, s_o, cn, carry, s_part);
-                for (uint32_t e = threadIdx.x; e < cn; e += 256) gs[cb + e] = s_o[e];
+            const U ref = seg_code<K, DESC>(ik[0]);
+            U diff = 0;
+#pragma unroll
+            for (int i = 0; i < ITEMS; i++)
+                if (i < IT && wbase + (uint32_t)i * 32u + lane < n) diff |= seg_code<K, DESC>(k[i]) ^ ref;
+            diff = block_or(diff);
+            SegPlan plan = seg_plan(diff, n, seg_min_passes<K>(),
+                                    [&](uint32_t sh) { return sampled(ik, n, sh); });
+            uint32_t shift = plan.shift;
+            for (uint32_t p = 0; p < plan.passes; p++) {
+                seg_rank_tile<K, DESC, ITEMS>(k, pos, IT, n, shift, s_whist, s_cnt, s_start, s_wsum);
+#pragma unroll
+                for (int i = 0; i < ITEMS; i++) {
+                    const uint32_t e = wbase + (uint32_t)i * 32u + lane;
+                    if (i < IT && e < n) { s_k[pos[i]] = k[i]; s_v[pos[i]] = v[i]; }
+                }
+                __syncthreads();
+                shift += 8u;
+                if (p + 1 == plan.passes) {
+                    if (plan.shift == 0 || sorted_runs(s_k, s_v, n, plan.shift)) break;
+                    plan = seg_full_plan(diff);
+                    shift = 0;
+                    p = ~0u;  // from the first pass again
+                }
+#pragma unroll
+                for (int i = 0; i < ITEMS; i++) {
+                    const uint32_t e = wbase + (uint32_t)i * 32u + lane;
+                    if (i < IT && e < n) { k[i] = s_k[e]; v[i] = s_v[e]; }
+                }
+                __syncthreads();
             }
-            __syncthreads();
+            // s_k / s_v hold the sorted segment; exclusive scan of the values into s_o
+            if (gs) seg_block_excl_scan<V, ITEMS>(s_v, s_o, n, first, s_part);
+            for (uint32_t e = threadIdx.x; e < n; e += 256) {
+                gk[st + e] = s_k[e];
+                gv[st + e] = s_v[e];
+                if (gs) gs[st + e] = s_o[e];
+            }
         }
     };
 
@@ -677,36 +1083,37 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
         unsigned long long base;
         fetch(item, gk, gv, gs, len, base);
         if (len == 0) continue;
-        if (len > (TRTC_SEG_GROUPS ? 4u : 1u) * WSEG) {
-            block_segment(gk, gv, gs, len, base);
-            continue;
-        }
-        // a small segment: the queue lists the classes from the largest down, so the entries
+        // a segment of the CTA classes is sorted by the whole CTA below (one copy of that code).
+        // A small one: the queue lists the classes from the largest down, so the entries
         // after it are no longer than its class.  The CTA splits into groups of G warps (one
         // warp up to WSEG keys, two up to 2 WSEG, four up to 4 WSEG), takes one more entry per
         // further group, and every group sorts one; an entry longer than its group's share
         // (list mode keeps the caller's order) is deferred to the whole CTA afterwards
         const uint32_t G = !TRTC_SEG_GROUPS ? 1u : len > 2u * WSEG ? 4u : (len > WSEG ? 2u : 1u);  // CTA-uniform
-        if (threadIdx.x == 0) s_batch = atomicAdd(&ctrl->next, (unsigned long long)(8u / G - 1u));
-        __syncthreads();
-        const uint32_t grp = warp / G;
-        const unsigned long long mine = grp == 0 ? item : s_batch + grp - 1;
-        unsigned long long defer = ~0ull;
-        if (mine < nseg) {
-            KB* wk;
-            V* wv;
-            V* ws;
-            uint32_t wl;
-            unsigned long long wb;
-            fetch(mine, wk, wv, ws, wl, wb);
-            if (wl > G * WSEG) defer = mine;
-            else if (wl > 0 && G == 1 && wl <= warp_small) seg_warp_bitonic<K, V, DESC>(wk, wv, ws, wl);
-            else if (wl > 0 && G == 1)
-                seg_warp_sort_scan<K, V, DESC, ITEMS>(wk, wv, ws, wl, s_k + warp * WSEG, s_v + warp * WSEG,
-                                                      s_whist + warp * 256);
-            else if (wl > 0)
-                seg_group_sort_scan<K, V, DESC, ITEMS>(wk, wv, ws, wl, s_k + grp * G * WSEG, s_v + grp * G * WSEG,
-                                                       s_o + grp * G * WSEG, s_whist, s_wsum, s_part, G, 1u + grp);
+        unsigned long long defer = warp == 0 ? item : ~0ull;
+        if (len <= (TRTC_SEG_GROUPS ? 4u : 1u) * WSEG) {  // CTA-uniform
+            if (threadIdx.x == 0) s_batch = atomicAdd(&ctrl->next, (unsigned long long)(8u / G - 1u));
+            __syncthreads();
+            const uint32_t grp = warp / G;
+            const unsigned long long mine = grp == 0 ? item : s_batch + grp - 1;
+            defer = ~0ull;
+            if (mine < nseg) {
+                KB* wk;
+                V* wv;
+                V* ws;
+                uint32_t wl;
+                unsigned long long wb;
+                fetch(mine, wk, wv, ws, wl, wb);
+                if (wl > G * WSEG) defer = mine;
+                else if (wl > 0 && G == 1 && wl <= warp_small) seg_warp_bitonic<K, V, DESC>(wk, wv, ws, wl);
+                else if (wl > 0 && G == 1)
+                    seg_warp_sort_scan<K, V, DESC, ITEMS>(wk, wv, wk, wv, ws, wl, V(), s_k + warp * WSEG,
+                                                          s_v + warp * WSEG, s_whist + warp * 256);
+                else if (wl > 0)
+                    seg_group_sort_scan<K, V, DESC, ITEMS>(wk, wv, wk, wv, ws, wl, V(), s_k + grp * G * WSEG,
+                                                           s_v + grp * G * WSEG, s_o + grp * G * WSEG, s_whist, s_wsum,
+                                                           s_part, G, 1u + grp);
+            }
         }
         if (lane == 0) s_defer[warp] = (warp % G == 0) ? defer : ~0ull;
         __syncthreads();
