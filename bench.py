@@ -72,7 +72,7 @@ WORKLOADS = {
                      "Gkeys/s Sort 2^27 f32 N(0,1) with -0.0, NaN, duplicates", "Gkeys/s"),
     "c3b_sort_by_key_i64_zipf": (1 << 27, "radix_pass_kernel", 24, 80,
                                  "Gkeys/s Sort_By_Key 2^27 i64 Zipf keys + i32 payload", "Gkeys/s"),
-    "c3c_copy_if_functor": (1 << 28, "jit:trtc::compact2_kernel", 6, 6,
+    "c3c_copy_if_functor": (1 << 28, "jit:trtc::compact_pipe_kernel", 6, 6,
                             "GB/s Copy_If 2^28 i32 with a user Functor (x & 1) != 0", "GB/s"),
     "c3d_scan_by_key_f32": (1 << 28, "scan_by_key_kernel", 12, 12,
                             "GB/s inclusive Scan_By_Key 2^28 f32 values, geometric runs", "GB/s"),
@@ -1188,7 +1188,7 @@ def run_mixed(args):
     per_launch_ms = statistics.mean(kt) if kt else None
     achieved = b_launch * n / (per_launch_ms / 1e3) / 1e9 if per_launch_ms else None
     if kname is None:
-        # a composed call (Reduce_By_Key: segmented scan + compaction): its algorithmic bytes
+        # Reduce_By_Key (its kernel and what initialises it): its algorithmic bytes
         # over the device time of all its kernels per call
         kname = "all kernels of the call"
         kt = [t for _, t in recs]
