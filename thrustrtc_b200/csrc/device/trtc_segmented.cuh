@@ -733,7 +733,7 @@ constexpr size_t seg_sort_scan_smem() {
 // in place); scan: receives the exclusive scans; tk/tv: temp arrays of n elements (large
 // segments only).
 // resident CTAs per SM the batched kernel is compiled for (B200, 100k lognormal segments at 8
-// items, u32 keys: 2 CTAs (127 registers) 4.15 ms, 3 CTAs 3.53 ms, 4 CTAs (64 registers) 3.46 ms;
+// items, u32 keys, all four passes per key: 2 CTAs (127 registers) 4.15 ms, 3 CTAs 3.53 ms, 4 CTAs (64 registers) 3.46 ms;
 // 16 items need the shared memory of 3 CTAs; 8-byte keys keep 2 CTAs, which they fill without
 // spilling)
 #ifndef TRTC_SEG_MINB
