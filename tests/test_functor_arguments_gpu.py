@@ -1,0 +1,62 @@
+"""A user's predicate is called on elements of the array only: it may index a captured vector by its
+argument.  The functors here check their arguments themselves, count those that are not what the
+call promises, and make no access with them."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def trtc(cuda):
+    import thrustrtc_b200 as t
+    t.init()
+    return t
+
+
+# the compaction pipeline starts at 2^22 elements; tiles of 5120 4-byte and 2560 8-byte elements
+EDGE = -(-(1 << 22) // 5120) * 5120
+SIZES = [1, 100, 5121, EDGE - 1, EDGE, EDGE + 1, EDGE + 20, EDGE + 2559, EDGE + 5119]
+BASE = 1 << 20  # elements are BASE + their index: zeros and foreign words are none of them
+
+
+def looked_up(trtc, n):
+    """table[x - BASE] behind a check of x; calls[] counts per element, bad[0] the arguments that are none."""
+    table = (np.arange(n) % 3 == 0).astype(np.int32)
+    calls, bad = trtc.device_vector_from_numpy(np.zeros(n, np.int32)), trtc.device_vector_from_numpy(np.zeros(1, np.int32))
+    f = trtc.Functor({"table": trtc.device_vector_from_numpy(table), "calls": calls, "bad": bad}, ["x"],
+                     "        long long i = (long long)x - %d;\n"
+                     "        if (i < 0 || i >= (long long)table.size()) { atomicAdd(&bad[0], 1); return false; }\n"
+                     "        atomicAdd(&calls[i], 1);\n"
+                     "        return table[i] != 0;\n" % BASE)
+    return f, table != 0, calls, bad
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+def test_selection_predicates(trtc, n, dtype):
+    x = np.arange(BASE, BASE + n).astype(dtype)
+    d, o, r = (trtc.device_vector_from_numpy(a) for a in (x, np.zeros(n, dtype), np.zeros(n, dtype)))
+    f, keep, calls, bad = looked_up(trtc, n)
+    assert trtc.Copy_If(d, o, f) == keep.sum() and o.to_host(0, int(keep.sum())).tobytes() == x[keep].tobytes()
+    assert trtc.Remove_Copy_If(d, o, f) == n - keep.sum()
+    if n > 1:
+        assert o.to_host(0, int(n - keep.sum())).tobytes() == x[~keep].tobytes()
+    assert trtc.Partition_Copy(d, o, r, f) == keep.sum()
+    assert bad.to_host()[0] == 0
+    c = calls.to_host()
+    assert c.min() >= 3 and c.min() == c.max()  # no element more often than another
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+def test_neighbour_predicate(trtc, n, dtype):
+    x = np.arange(BASE, BASE + n).astype(dtype)
+    d, o = trtc.device_vector_from_numpy(x), trtc.device_vector_from_numpy(np.zeros(n, dtype))
+    bad = trtc.device_vector_from_numpy(np.zeros(1, np.int32))
+    f = trtc.Functor({"bad": bad, "n": trtc.DVInt32(n)}, ["a", "b"],
+                     "        if (a != b + 1 || b < %d || a >= %d + n) { atomicAdd(&bad[0], 1); return false; }\n"
+                     "        return a / 2 == b / 2;\n" % (BASE, BASE))
+    heads = np.concatenate([[True], x[1:] // 2 != x[:-1] // 2])
+    assert trtc.Unique_Copy(d, o, f) == heads.sum() and o.to_host(0, int(heads.sum())).tobytes() == x[heads].tobytes()
+    assert bad.to_host()[0] == 0

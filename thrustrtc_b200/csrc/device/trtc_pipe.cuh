@@ -761,27 +761,39 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
             }
             E x[ITEMS];
             pipe_load_run<E, ITEMS>(p + t0, x);
+            const uint32_t left = cnt > t0 ? cnt - t0 : 0u;  // this thread's elements
+            auto test = [&](const E& v, const E& prev) -> bool {
+                if constexpr (MODE == CM_PRED) return (bool)pred(v);
+                else if constexpr (MODE == CM_NOT_EQUAL) return !(v == value);
+                else if constexpr (MODE == CM_NOT_PRED) return !(bool)pred(v);
+                else if constexpr (MODE == CM_UNIQUE) return v != prev;
+                else return !(bool)pred(v, prev);
+            };
+            // A user's predicate is called on elements of the array only: it may index by its argument.
+            // The last tile, and tile 0 where the neighbour is tested, take a loop over what there is; the
+            // tiles between, all of whose elements (and neighbours) exist, an unrolled one without tests.
+            const bool whole = cnt == TILE && !(NEIGH && tile == 0);
+            uint32_t sel = 0;
+            if (!whole) {
+                const uint32_t end = left < (uint32_t)ITEMS ? left : (uint32_t)ITEMS;
+#pragma unroll 1
+                for (uint32_t j = 0; j < end; j++) {
+                    const E* e = p + t0 + j;
+                    if ((NEIGH && tile == 0 && t0 + j == 0) || test(*e, NEIGH ? e[-1] : *e)) sel |= 1u << j;
+                }
+            }
             E before = E();
             if constexpr (NEIGH) {
                 before = shfl_up_any(x[ITEMS - 1], 1);
-                if (lane == 0) before = p[(int)t0 - 1];
+                if (lane == 0 && whole) before = p[(int)t0 - 1];
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars.empty[s]);
-            uint32_t sel = 0;
+            if (whole) {
 #pragma unroll
-            for (int j = 0; j < ITEMS; j++) {
-                bool f;
-                if constexpr (MODE == CM_PRED) f = (bool)pred(x[j]);
-                else if constexpr (MODE == CM_NOT_EQUAL) f = !(x[j] == value);
-                else if constexpr (MODE == CM_NOT_PRED) f = !(bool)pred(x[j]);
-                else if constexpr (MODE == CM_UNIQUE) f = x[j] != (j == 0 ? before : x[j > 0 ? j - 1 : 0]);
-                else f = !(bool)pred(x[j], j == 0 ? before : x[j > 0 ? j - 1 : 0]);
-                if (f) sel |= 1u << j;
+                for (int j = 0; j < ITEMS; j++)
+                    if (test(x[j], j == 0 ? before : x[j > 0 ? j - 1 : 0])) sel |= 1u << j;
             }
-            if (NEIGH && tile == 0 && gt == 0) sel |= 1u;
-            const uint32_t left = cnt > t0 ? cnt - t0 : 0u;  // this thread's elements
-            if (left < (uint32_t)ITEMS) sel &= (1u << left) - 1u;
             const uint32_t mine = (uint32_t)__popc(sel);
             const uint32_t c = pipe_lane_sums<32>(mine);
             if (lane == 31) s_wcnt[b][gw] = c;
