@@ -60,3 +60,26 @@ def test_neighbour_predicate(trtc, n, dtype):
     heads = np.concatenate([[True], x[1:] // 2 != x[:-1] // 2])
     assert trtc.Unique_Copy(d, o, f) == heads.sum() and o.to_host(0, int(heads.sum())).tobytes() == x[heads].tobytes()
     assert bad.to_host()[0] == 0
+
+
+@pytest.mark.parametrize("n", [1, 2, 20, 2560, 2561, 5119, 5120, 5121, 5140, 10240, 20_483, EDGE + 7])
+@pytest.mark.parametrize("dtype", [np.int16, np.int32, np.int64])
+def test_key_predicate(trtc, n, dtype):
+    # keys count up (modulo a range above zero): neighbours, or a key and itself, and nothing else
+    m = min(n, 30_000)
+    base = 1000 if dtype == np.int16 else BASE
+    k = (base + np.arange(n) % m).astype(dtype)
+    dk, dv = trtc.device_vector_from_numpy(k), trtc.device_vector_from_numpy(np.ones(n, np.int32))
+    ko, vo = trtc.device_vector_from_numpy(np.zeros(n, dtype)), trtc.device_vector_from_numpy(np.zeros(n, np.int32))
+    bad = trtc.device_vector_from_numpy(np.zeros(1, np.int32))
+    f = trtc.Functor({"bad": bad, "m": trtc.DVInt32(m)}, ["a", "b"],
+                     "        long long i = (long long)a - %d, j = (long long)b - %d;\n"
+                     "        if (i < 0 || i >= m || (j != (i + 1) %% m && j != i)) { atomicAdd(&bad[0], 1); return false; }\n"
+                     "        return i / 2 == j / 2;\n" % (base, base))
+    i = np.arange(n) % m
+    heads = np.flatnonzero(np.concatenate([[True], (i[1:] // 2 != i[:-1] // 2)]))
+    last = np.concatenate([heads[1:] - 1, [n - 1]])
+    assert trtc.Reduce_By_Key(dk, dv, ko, vo, f) == len(heads)
+    assert bad.to_host()[0] == 0
+    assert ko.to_host(0, len(heads)).tobytes() == k[last].tobytes()
+    assert vo.to_host(0, len(heads)).tobytes() == (last - heads + 1).astype(np.int32).tobytes()

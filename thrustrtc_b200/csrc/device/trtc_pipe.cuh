@@ -453,11 +453,21 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
                     vp[i] = (E)vals[base + i];
                 }
                 if (gt == 0 && base > 0) kp[-1] = (K)keys[base - 1];
-                if (gt == 1 && base + cnt < n) kp[cnt] = (K)keys[base + cnt];
+                if (base + cnt < n) {
+                    if (gt == 1) kp[cnt] = (K)keys[base + cnt];
+                } else {
+                    // no key behind the last: itself stands in (see tile 0)
+                    const K last = (K)keys[n - 1];
+                    for (uint32_t i = cnt + gt; i <= TILE; i += GT) kp[i] = last;
+                }
             } else if (!VTMA) {
                 for (uint32_t i = gt; i < TILE; i += GT) vp[i] = (E)vals[base + i];
             }
-            if (!bulk || !VTMA) {
+            // A user's predicate may index by the keys, so it only ever sees keys of the array: where a
+            // neighbour is missing (its answer is not used) the key itself is put in the stage.  Tests
+            // around the calls instead split the fold's straight line: 50 M elements 99.9 us per call, this way 95.8.
+            if (tile == 0 && gt == 0) kp[-1] = (K)keys[0];
+            if (!bulk || !VTMA || tile == 0) {
                 // these writes come before a later bulk copy into the stage
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 pipe_sync(bar, GT);
