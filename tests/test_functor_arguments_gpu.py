@@ -83,3 +83,27 @@ def test_key_predicate(trtc, n, dtype):
     assert bad.to_host()[0] == 0
     assert ko.to_host(0, len(heads)).tobytes() == k[last].tobytes()
     assert vo.to_host(0, len(heads)).tobytes() == (last - heads + 1).astype(np.int32).tobytes()
+
+
+@pytest.mark.parametrize("n", [1, 5121, 300_000, 8_000_003])
+@pytest.mark.parametrize("run", [3, 7000, 1 << 30])
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+def test_value_operator(trtc, n, run, dtype):
+    # values from one range under an operator that is only defined on it; the call before leaves other
+    # words in the stream's workspace
+    k = (np.arange(n) // run).astype(np.int32)
+    v = (BASE + (np.arange(n) * 2654435761 >> 7) % 5000).astype(dtype)
+    dk, dv = trtc.device_vector_from_numpy(k), trtc.device_vector_from_numpy(v)
+    ko, vo = trtc.device_vector_from_numpy(np.zeros(n, np.int32)), trtc.device_vector_from_numpy(np.zeros(n, dtype))
+    bad = trtc.device_vector_from_numpy(np.zeros(1, np.int32))
+    f = trtc.Functor({"bad": bad}, ["a", "b"],
+                     "        if (a < %d || a >= %d || b < %d || b >= %d) atomicAdd(&bad[0], 1);\n"
+                     "        return a > b ? a : b;\n" % (BASE, BASE + 5000, BASE, BASE + 5000))
+    heads = np.arange(0, n, run)
+    want = np.maximum.reduceat(v, heads).astype(dtype)
+    minus = trtc.device_vector_from_numpy(np.full(n, -7, dtype))
+    for _ in range(5):
+        trtc.Reduce_By_Key(dk, minus, ko, vo, trtc.EqualTo(), trtc.Minimum())
+        assert trtc.Reduce_By_Key(dk, dv, ko, vo, trtc.EqualTo(), f) == len(heads)
+        assert vo.to_host(0, len(heads)).tobytes() == want.tobytes()
+    assert bad.to_host()[0] == 0

@@ -147,13 +147,14 @@ __device__ void pipe_prefix_scan(const LookbackState& st, const LookbackState& a
             fence_acq_rel();
             if (f) v = reinterpret_cast<const T*>(st.agg)[j];
         }
-        // inclusive scan over the lanes (values behind the gap reach no lane before it)
+        // inclusive scan over the lanes before the gap (op only ever sees what was published: behind
+        // the gap v is T(), or what an earlier call left in the word)
         const uint32_t hm = SEG ? __ballot_sync(0xffffffffu, (f & 4u) != 0u) : 0u;
         T vi = v;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const T vy = shfl_up_any(vi, d);
-            if (lane >= (uint32_t)d) {
+            if (lane >= (uint32_t)d && lane < lead) {
                 const uint32_t win = le & ~((1u << (lane - (uint32_t)d + 1u)) - 1u);
                 if ((hm & win) == 0u) vi = (T)op(vy, vi);
             }
@@ -177,7 +178,7 @@ __device__ void pipe_prefix_scan(const LookbackState& st, const LookbackState& a
 #pragma unroll
             for (int d = 1; d < 16; d <<= 1) {
                 const T y = shfl_up_any(w, d);
-                if (lane >= (uint32_t)d) {
+                if (lane >= (uint32_t)d && in) {
                     const uint32_t win = le & ~((1u << (lane - (uint32_t)d + 1u)) - 1u);
                     if ((wh & win) == 0u) w = (T)op(y, w);
                 }
@@ -185,11 +186,11 @@ __device__ void pipe_prefix_scan(const LookbackState& st, const LookbackState& a
             // what precedes the warp's first tile
             const T y = shfl_up_any(w, 1);
             const bool yhd = (wh & (le >> 1)) != 0u;
+            const uint32_t nin = (uint32_t)__popc(inm);  // (lanes 0 to nin - 1)
             T pre = run;
-            if (lane > 0) pre = (yhd || !run_h) ? y : (T)op(run, y);
+            if (lane > 0 && in) pre = (yhd || !run_h) ? y : (T)op(run, y);
             s_v[lane] = pre;
             s_has[lane] = run_h || lane > 0 ? 1u : 0u;
-            const uint32_t nin = (uint32_t)__popc(inm);
             if (nin && lane == nin - 1u) s_total = ((wh & le) != 0u || !run_h) ? w : (T)op(run, w);
             const uint32_t t = __reduce_add_sync(0xffffffffu, in ? l : 0u);
             s_lead[lane] = in ? l : 0u;
