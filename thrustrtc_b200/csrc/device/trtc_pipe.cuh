@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
             if (tile == 0 && gt == 0) kp[-1] = (K)keys[0];
             if (!bulk || !VTMA || tile == 0) {
                 // these writes come before a later bulk copy into the stage
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                smem_proxy_fence();
                 pipe_sync(bar, GT);
             }
             K kk[ITEMS];
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
                 for (uint32_t i = gt; i < cnt; i += GT) p[i] = in[base + i];
                 if (NEIGH && gt == 0 && base > 0) p[-1] = in[base - 1];
                 // these writes come before a later bulk copy into the stage
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                smem_proxy_fence();
                 pipe_sync(bar, GT);
             }
             E x[ITEMS];
@@ -988,7 +988,7 @@ __global__ void __launch_bounds__(PipeShape<SpipeShape<K, T>::G>::THREADS, 1) sc
                     vp[i] = vals[base + i];
                 }
                 if (gt == 0 && base > 0) kp[-1] = keys[base - 1];
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                smem_proxy_fence();
                 pipe_sync(bar, GT);
             }
             K kk[ITEMS];

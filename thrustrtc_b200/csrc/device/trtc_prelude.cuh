@@ -139,10 +139,12 @@ TRTC_FORCEINLINE uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_gene
 TRTC_FORCEINLINE void mbar_init(unsigned long long* bar, uint32_t arrivals) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(arrivals) : "memory");
 }
+// this thread's ordinary shared-memory accesses before copies that the engine starts after a barrier
+TRTC_FORCEINLINE void smem_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 // makes initialised barriers visible to the copy engine (async proxy)
 TRTC_FORCEINLINE void mbar_init_fence() {
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    smem_proxy_fence();
 }
 TRTC_FORCEINLINE void mbar_init_one(unsigned long long* bar) {
     mbar_init(bar, 1u);

@@ -739,6 +739,9 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     if (gridDim.x >= tiles) return;  // a tile per CTA
     vphase ^= vbulk ? 1u : 0u;
     if (EARLY && threadIdx.x == 0) s_tile = next;
+    // this tile's ordinary stores to s_vals come before the next tile's bulk copy into it (another
+    // proxy, which the barrier alone does not order)
+    if constexpr (VB) smem_proxy_fence();
     __syncthreads();
     }
 }
