@@ -129,6 +129,16 @@ int trtc_raw_segmented_tuning_load(const char* json);
  * trtc_last_error(), and the library stays usable (out holds garbage).  Synchronous. */
 int trtc_test_scan_lookback_timeout(const int* in, int* out, unsigned long long n, void* stream);
 
+/* test hook (csrc/host/launch_single_cta.cu): the tile pipeline's kernels in grids of `ctas` CTAs (1: the prefix
+ * CTA alone, as when another stream's kernel leaves room for one).  what: 0 odd elements of in to out and
+ * the others to out2, 1 unique, 2 inclusive scan by key, 3 exclusive scan by key behind 5, 4 reduce by
+ * key (sums to out, keys to out2).  All arrays hold n elements on the device; *count: results, ~0 when 0, 1 or 4
+ * gave up before it began because the prefix CTA was alone.  Synchronous. */
+int trtc_test_pipe_few_ctas(int what, unsigned ctas, int* keys, int* in, int* out, int* out2, unsigned long long n,
+                            unsigned long long* count, void* stream);
+/* test hook: `ctas` CTAs of 32 threads that hold `smem` bytes of shared memory for `micros` (<= 10^6) microseconds */
+int trtc_test_occupy(unsigned ctas, unsigned smem, unsigned micros, void* stream);
+
 /* diagnostics: copies the sort control block of the last sort on `stream` */
 unsigned long long trtc_debug_sort_ctrl(void* host, unsigned long long bytes, void* stream);
 

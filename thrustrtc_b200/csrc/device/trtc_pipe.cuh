@@ -16,7 +16,10 @@
 //   store warps       write the staged results at their final place (a tile each).
 // One CTA of the grid, the prefix CTA, scans what the tiles publish (half of its warps the counts,
 // half the running values where there are any) and answers every tile with what precedes it.  Tickets are drawn in
-// order by running CTAs, so a tile only ever waits for tiles that are under way.
+// order by running CTAs, so a tile only ever waits for tiles that are under way.  A worker that runs
+// draws until the end.  When none does (a long kernel of another stream leaves room for the prefix CTA
+// only), calls that read a result back give up before the first tile and the host takes the general form;
+// the scan, whose call has returned by then, does tiles in the prefix CTA.
 //
 // Every wait is bounded: a role whose wait expires records the error and leaves, the others
 // follow (their waits see the error word), and the producer draws its remaining tickets so
@@ -29,7 +32,9 @@ namespace trtc {
 enum : int {
     PIPE_COMPUTE = 8,   // warps of a compute group
     PIPE_STORE = 4,     // store warps
-    PIPE_META = 16      // tiles of a CTA between folding and stored, at most
+    PIPE_META = 16,     // tiles of a CTA between folding and stored, at most
+    PIPE_ALONE = 1024   // polls (about 1 ms; workers draw within microseconds of their start) before the
+                        // prefix CTA takes itself to be alone
 };
 template <int G> struct PipeShape {
     enum : int { WARPS = PIPE_COMPUTE * G + PIPE_STORE + 3, THREADS = WARPS * 32 };
@@ -116,6 +121,92 @@ TRTC_FORCEINLINE void pipe_await_slots(unsigned long long* agg, unsigned long lo
     }
 }
 
+// Alone before the first tile: takes all tickets, so that workers that come later leave at once, and
+// reports ~0 as the call's result.  `gone` (shared memory, zero) tells the other half of the CTA, whose
+// own PipeCancel has no result.
+struct PipeCancel {
+    unsigned long long* ctr;
+    uint32_t tiles;
+    volatile uint32_t* gone;
+    unsigned long long* result;
+    TRTC_FORCEINLINE bool now(uint32_t first, uint32_t spins) {
+        if (!result) return *gone != 0u;
+        const unsigned long long end = (unsigned long long)tiles + 1u;
+        if (first > 0u || spins < (uint32_t)PIPE_ALONE || atomicCAS(ctr, 1ull, end) != 1ull) return false;
+        if (gridDim.x == 1) atomicExch(ctr, 0ull);  // (no worker to draw the last ticket)
+        *result = ~0ull;
+        *gone = 1u;
+        return true;
+    }
+    template <class T> TRTC_FORCEINLINE bool act(uint32_t, const T&, bool) { return false; }
+};
+
+// Alone at any tile: draws it (draw(tile): false when somebody else has) and does it (tile_alone).
+template <class Draw, class Tile> struct PipeSolo {
+    Draw draw;
+    Tile tile_alone;
+    uint32_t patience = PIPE_ALONE;
+    TRTC_FORCEINLINE bool now(uint32_t first, uint32_t spins) {
+        if (spins < patience) return false;
+        const bool mine = draw(first);
+        patience = mine ? 8u : (uint32_t)PIPE_ALONE;
+        return mine;
+    }
+    template <class T> TRTC_FORCEINLINE bool act(uint32_t first, const T& run, bool run_h) {
+        tile_alone(first, run, run_h);
+        return true;
+    }
+};
+
+// What the prefix CTA needs to do a tile itself, one element per thread of WARPS warps at a time (no
+// stages: the prefix is known).  The elements of a chunk are those of its first threads.
+// PipeRun: what a tile has come to before a chunk: its running value (when there is one), and whether no head
+// stood in it so far.
+template <class T> struct PipeRun {
+    T v = T();
+    bool has = false, open = true;
+};
+template <class T, int WARPS> struct PipeChunk {
+    T v[WARPS];
+    uint32_t has[WARPS], head[WARPS];
+};
+// inclusive segmented scan behind `run`, which moves on past the chunk; open: no head in the tile up to
+// this thread's element
+template <int WARPS, class T, class Op>
+TRTC_FORCEINLINE T pipe_chunk_scan(T v, bool head, bool valid, Op& op, uint32_t warp, uint32_t bar,
+                                   PipeChunk<T, WARPS>* s, PipeRun<T>& run, bool& open) {
+    const uint32_t lane = lane_id(), le = lane == 31u ? 0xffffffffu : ((2u << lane) - 1u);
+    const uint32_t vm = __ballot_sync(0xffffffffu, valid), hm = __ballot_sync(0xffffffffu, valid && head);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const T y = shfl_up_any(v, d);
+        if (valid && lane >= (uint32_t)d) {
+            const uint32_t win = le & ~((1u << (lane - (uint32_t)d + 1u)) - 1u);
+            if ((hm & win) == 0u) v = (T)op(y, v);
+        }
+    }
+    if (vm && lane == 31u - (uint32_t)__clz(vm)) s->v[warp] = v;
+    if (lane == 0) {
+        s->has[warp] = vm != 0u;
+        s->head[warp] = hm != 0u;
+    }
+    pipe_sync(bar, WARPS * 32);
+    open = false;
+#pragma unroll 1
+    for (uint32_t w = 0; w < (uint32_t)WARPS; w++) {
+        if (w == warp) {
+            if (valid && (hm & le) == 0u && run.has) v = (T)op(run.v, v);
+            open = run.open && (hm & le) == 0u;
+        }
+        if (!s->has[w]) continue;
+        run.v = (s->head[w] || !run.has) ? s->v[w] : (T)op(run.v, s->v[w]);
+        run.has = true;
+        run.open = run.open && !s->head[w];
+    }
+    pipe_sync(bar, WARPS * 32);  // s is free
+    return v;
+}
+
 // Half of the prefix CTA: polls one tile per thread from the first unanswered one on, takes in the published
 // ones that follow without a gap, scans them across the CTA and answers each with what precedes
 // it (SEG: a segmented scan, a head discards what is before it).  Tiles then poll a single word
@@ -124,9 +215,11 @@ TRTC_FORCEINLINE void pipe_await_slots(unsigned long long* agg, unsigned long lo
 // took 150 to 210 us where they take 88 us without any wait for prefixes.
 // WARPS warps from warp0 on run one stream of values, published in st, answered in `answers` (the same
 // words, or others); bar: a barrier of their own.
-template <class T, class Op, bool SEG, int WARPS>
+// alone: what to do while no other CTA runs (PipeCancel, or a kernel's own).  alone.now(first, spins), by one
+// thread after a poll without progress: is it time?  Then alone.act(first, run, run_h), by all: false to leave.
+template <class T, class Op, bool SEG, int WARPS, class Alone>
 __device__ void pipe_prefix_scan(const LookbackState& st, const LookbackState& answers, uint32_t tiles, Op& op,
-                                 unsigned long long* result, uint32_t warp0, uint32_t bar) {
+                                 unsigned long long* result, uint32_t warp0, uint32_t bar, Alone alone) {
     static_assert(WARPS <= 16, "one scan of 16 warps");
     __shared__ uint32_t s_lead[32], s_hd[32], s_has[32], s_taken;
     __shared__ T s_v[32], s_total;
@@ -212,11 +305,15 @@ __device__ void pipe_prefix_scan(const LookbackState& st, const LookbackState& a
             run_h = true;
             spins = 0;
         }
-        bool give_up = false;
-        if (!taken) give_up = !spin_continue(spins, st.err);
-        if (pipe_any(bar, WARPS * 32, give_up)) {
-            report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
-            return;
+        bool give_up = false, act = false;
+        if (!taken) {
+            give_up = !spin_continue(spins, st.err);
+            act = thread == 0 && alone.now(first, spins);
+        }
+        if (pipe_any(bar, WARPS * 32, give_up || act)) {
+            const bool fail = pipe_any(bar, WARPS * 32, give_up);
+            if (fail) report_error(st.err, TRTC_ERR_LOOKBACK_TIMEOUT);
+            if (fail || !alone.act(first, run, run_h)) return;
         }
         first += taken;
     }
@@ -397,6 +494,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
     __shared__ T s_wtot[2 * G][PIPE_COMPUTE];
     __shared__ __align__(16) uint32_t s_wcnt[2 * G][PIPE_COMPUTE];  // results of the warp's elements, bit 31: holds a head
     __shared__ uint32_t m_last;  // the CTA's number of tiles, once known
+    __shared__ uint32_t s_gone;  // (prefix CTA)
     __shared__ unsigned long long s_first;
 
     const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
@@ -405,6 +503,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
     RbkResult<K, T>* ring = reinterpret_cast<RbkResult<K, T>*>(pipe_smem + SM::RING);
     if (threadIdx.x == 0) bars.init(2u);
     if (threadIdx.x == 0) m_last = 0xFFFFFFFFu;
+    if (threadIdx.x == 0) s_gone = 0u;
     if (threadIdx.x < 2 * PIPE_META) m_stored[threadIdx.x] = 0;
     // tickets: the first one makes its CTA the prefix CTA (running before any tile can wait for it),
     // ticket t > 0 is tile t - 1; every other CTA draws until it holds one past the last tile
@@ -413,10 +512,13 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
     if (s_first == 0) {
         constexpr int HALF = PipeShape<G>::WARPS / 2;
         Plus plus;
+        unsigned long long* result = reinterpret_cast<unsigned long long*>(st.result);
         if (warp < HALF)
-            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, st, tiles, plus, reinterpret_cast<unsigned long long*>(st.result), 0u, 1u);
+            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, st, tiles, plus, result, 0u, 1u,
+                                                          PipeCancel{st.tile_ctr, tiles, &s_gone, result});
         else if (warp < 2 * HALF)
-            pipe_prefix_scan<T, Op, true, HALF>(st2, st2, tiles, op, nullptr, HALF, 2u);
+            pipe_prefix_scan<T, Op, true, HALF>(st2, st2, tiles, op, nullptr, HALF, 2u,
+                                                PipeCancel{st.tile_ctr, tiles, &s_gone, nullptr});
         return;
     }
     constexpr uint32_t GT = PIPE_COMPUTE * 32;  // threads of a group
@@ -718,6 +820,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
     __shared__ uint32_t m_end[2 * PIPE_META], m_stored[2 * PIPE_META];  // as in rbk_pipe_kernel
     __shared__ uint32_t s_wcnt[2 * G][PIPE_COMPUTE];
     __shared__ uint32_t m_last;
+    __shared__ uint32_t s_gone;  // (prefix CTA)
     __shared__ unsigned long long s_first;
 
     const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
@@ -726,6 +829,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
     if (threadIdx.x == 0) {
         bars.init(1u);
         m_last = 0xFFFFFFFFu;
+        s_gone = 0u;
         s_first = atomicAdd(st.tile_ctr, 1ull);
     }
     if (threadIdx.x < 2 * PIPE_META) m_stored[threadIdx.x] = 0;
@@ -733,8 +837,10 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
     if (s_first == 0) {
         constexpr int HALF = PipeShape<G>::WARPS / 2;
         Plus plus;
+        unsigned long long* result = reinterpret_cast<unsigned long long*>(st.result);
         if (warp < HALF)
-            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, st, tiles, plus, reinterpret_cast<unsigned long long*>(st.result), 0u, 1u);
+            pipe_prefix_scan<uint32_t, Plus, false, HALF>(st, st, tiles, plus, result, 0u, 1u,
+                                                          PipeCancel{st.tile_ctr, tiles, &s_gone, result});
         return;
     }
     constexpr uint32_t GT = PIPE_COMPUTE * 32;  // threads of a group
@@ -955,7 +1061,49 @@ __global__ void __launch_bounds__(PipeShape<SpipeShape<K, T>::G>::THREADS, 1) sc
     Plus op;
     if (s_first == 0) {
         constexpr int HALF = PipeShape<G>::WARPS / 2;
-        if (warp < HALF) pipe_prefix_scan<T, Plus, true, HALF>(st, st2, tiles, op, nullptr, 0u, 1u);
+        // with no other CTA: a tile by this half's warps, whenever all drawn ones are answered (their next
+        // ticket is then this tile's) and nobody has drawn for a while; again soon after it
+        auto tile_alone = [&](uint32_t tile, const T& carry, bool has) {
+            auto* s_chunk = reinterpret_cast<PipeChunk<T, HALF>*>(pipe_smem);
+            T* s_x = reinterpret_cast<T*>(pipe_smem + 8192);
+            const size_t base = (size_t)tile * TILE;
+            const uint32_t cnt = (n - base) < (size_t)TILE ? (uint32_t)(n - base) : TILE;
+            PipeRun<T> run;
+            for (uint32_t c0 = 0; c0 < cnt; c0 += HALF * 32) {
+                const size_t i = base + c0 + threadIdx.x;
+                const bool valid = c0 + threadIdx.x < cnt;
+                T v = T();
+                bool head = false, open;
+                if (valid) {
+                    v = vals[i];
+                    head = i == 0 || !(keys[i] == keys[i - 1]);
+                }
+                T before = run.v;
+                v = pipe_chunk_scan<HALF>(v, head, valid, op, warp, 1u, s_chunk, run, open);
+                if constexpr (MODE == 1) {
+                    s_x[threadIdx.x] = v;
+                    pipe_sync(1u, HALF * 32);
+                    if (threadIdx.x > 0) before = s_x[threadIdx.x - 1];
+                    pipe_sync(1u, HALF * 32);
+                    if (i == base) before = carry;
+                    else if (open && has) before = (T)op(carry, before);
+                    v = head ? init : (T)op(init, before);
+                } else {
+                    if (open && has) v = (T)op(carry, v);
+                }
+                if (valid) out[i] = v;
+            }
+            if (threadIdx.x == 0) pipe_put<T>(st, tile, run.v, run.open ? 1u : 5u);
+        };
+        auto draw = [&](uint32_t tile) -> bool {
+            const unsigned long long t = (unsigned long long)tile + 1u;
+            if (atomicCAS(st.tile_ctr, t, t + 1u) != t) return false;
+            if (t == (unsigned long long)tiles + gridDim.x - 1) atomicExch(st.tile_ctr, 0ull);
+            return true;
+        };
+        if (warp < HALF)
+            pipe_prefix_scan<T, Plus, true, HALF>(st, st2, tiles, op, nullptr, 0u, 1u,
+                                                  PipeSolo<decltype(draw), decltype(tile_alone)>{draw, tile_alone});
         return;
     }
     constexpr uint32_t GT = PIPE_COMPUTE * 32;  // threads of a group

@@ -358,7 +358,7 @@ static bool compact_t(const T* in, T* out, size_t n, const T* value, cudaStream_
             if (!hr.dev() && !TRTC_CUDA(cudaMemcpyAsync(count, st.result, 8, cudaMemcpyDeviceToHost, s))) return false;
             if (!check_device_errors(s, "compaction")) return false;
             if (hr.dev()) hr.read(count, 8);
-            return true;
+            if (*count != ~0ull) return true;  // else it had no room to run (PipeCancel) and did nothing
         }
     }
     // the vector path (4-byte elements: remove's element-wise test, unique's neighbour test)

@@ -608,7 +608,7 @@ unsigned long long run_compact(CompactSpec& c) {
         if (!hr.dev() && !TRTC_CUDA(cudaMemcpyAsync(&cnt, lst.result, 8, cudaMemcpyDeviceToHost, S()))) return kFail;
         if (!check_device_errors(S(), "compaction")) return kFail;
         if (hr.dev()) hr.read(&cnt, 8);
-        return cnt;
+        if (cnt != ~0ull) return cnt;  // else it had no room to run (PipeCancel) and did nothing
     }
     // the 16-byte vector path (contiguous 4-byte input and output: element-wise tests of one
     // array, or neighbour tests with an optional second array) takes 32 items per thread; the
@@ -802,7 +802,7 @@ static bool cannot_overlap(const DVVectorLike& w, const DVVectorLike& r) {
 // staged results fill an SM's shared memory): tiles of 5120 elements of up to 8 bytes of key and
 // value, of 2560 up to 16.  20 and 10 elements per thread are 5 times 16 bytes of the widest
 // array: an odd number, so that the threads' 16-byte shared-memory loads do not share banks.
-// false: not this form (nothing was launched).
+// false: not this form, or no room for it on the GPU (PipeCancel); nothing was done.
 static bool reduce_by_key_pipe(const DVVectorLike& key_in, const DVVectorLike& value_in, DVVectorLike& key_out,
                                DVVectorLike& value_out, const Functor& pred, const Functor& op, uint32_t& count) {
     const size_t n = key_in.size();
@@ -854,6 +854,7 @@ static bool reduce_by_key_pipe(const DVVectorLike& key_in, const DVVectorLike& v
                       (hr.dev() || TRTC_CUDA(cudaMemcpyAsync(&cnt, w->result, 8, cudaMemcpyDeviceToHost, S()))) &&
                       check_device_errors(S(), "reduce_by_key");
     if (done && hr.dev()) hr.read(&cnt, 8);
+    if (done && cnt == ~0ull) return false;
     count = done ? to_u32(cnt) : (uint32_t)(-1);
     return true;
 }
