@@ -234,7 +234,10 @@ __global__ void __launch_bounds__(BLOCK) merge_level_kernel(const K* __restrict_
     // runs at the end (two sequential streams)
     constexpr bool SV = HAS_VALS && sizeof(K) <= 4 && sizeof(V) <= 4;
     __shared__ __align__(16) K s_k[T + 1];
-    __shared__ V s_v[SV ? T : 1];
+    // (bytes: aligned for 4-byte asynchronous copies whatever V's own alignment is, and without V's
+    // constructor, which a shared variable may not have)
+    __shared__ __align__(16) unsigned char s_vbytes[SV ? T * sizeof(V) : 16];
+    V* const s_v = reinterpret_cast<V*>(s_vbytes);
     __shared__ __align__(16) unsigned short s_from[T];
     __shared__ size_t s_path[2];
     typedef typename remove_cvref<typename OKV::value_t>::type OK;
