@@ -136,9 +136,10 @@ static bool radix_sort_run(K* keys, V* vals0, size_t n, cudaStream_t s, int vals
         // 5.739 ms without, 5.585 ms at 222 tiles, within 0.2 % from 148 to 444 tiles, slower
         // again past one wave of resident CTAs as the prefetched tiles crowd L2)
         const uint32_t pf = tile_prefetch_ahead((size_t)sms * 3 / 2);
-        static int per_sm = 0;
-        if (per_sm == 0 && (!TRTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel, BLOCK, smem)) || per_sm < 1))
-            per_sm = 1;
+        static const int per_sm = [&] {  // (once, whichever thread sorts first)
+            int v = 0;
+            return TRTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, pass_kernel, BLOCK, smem)) && v > 0 ? v : 1;
+        }();
         const size_t pgrid = (size_t)per_sm * sms < tiles ? (size_t)per_sm * sms : tiles;
         for (int p = 0; p < D; p++) {
             launch_dependent(pass_kernel, (unsigned)pgrid, BLOCK, smem, s, bufs, n, ctrl, p, (ST*)st0, (ST*)st1,
