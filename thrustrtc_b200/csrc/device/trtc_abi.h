@@ -19,4 +19,7 @@ struct LookbackState {
                                     // prefetches tile t + pf_ahead into L2 (0: none)
 };
 
+// dynamic shared memory that a tile pipeline kernel may use (with its static part within an SM's 227 KB)
+enum : unsigned { PIPE_SMEM = 220 * 1024 };
+
 }  // namespace trtc

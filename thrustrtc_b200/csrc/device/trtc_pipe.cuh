@@ -454,6 +454,7 @@ template <class K, class E, class T, int ITEMS, int S, int C> struct RbkSmem {
     static constexpr size_t STAGE = KEY_BYTES + ((size_t)TILE * sizeof(E) + 15) / 16 * 16;
     static constexpr size_t RING = S * STAGE;
     static constexpr size_t BYTES = RING + (size_t)(C + TILE) * sizeof(RbkResult<K, T>);
+    static_assert(BYTES <= PIPE_SMEM, "the launch's shared memory");
 };
 
 // B200, 50,000,011 int32 keys in runs of mean 32 with float sums: 85-90 us per launch (4.4 TB/s,
@@ -789,7 +790,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) rbk_pipe_kernel(KV k
 template <class E> struct CpipeShape {
     static constexpr int G = 3, ITEMS = 80 / (int)sizeof(E), S = 3;
     static constexpr int TILE = PIPE_COMPUTE * 32 * ITEMS;
-    static constexpr int RING = ((220 * 1024 - S * (TILE * (int)sizeof(E) + 16)) / (int)sizeof(E) - TILE) / 16 * 16;
+    static constexpr int RING = (((int)PIPE_SMEM - S * (TILE * (int)sizeof(E) + 16)) / (int)sizeof(E) - TILE) / 16 * 16;
     static constexpr size_t SMEM = S * ((size_t)TILE * sizeof(E) + 16) + (size_t)(RING + TILE) * sizeof(E);
 };
 template <class E, int ITEMS, int S> struct CpipeSmem {
@@ -812,6 +813,7 @@ __global__ void __launch_bounds__(PipeShape<G>::THREADS, 1) compact_pipe_kernel(
     constexpr uint32_t TILE = SM::TILE;
     constexpr bool NEIGH = MODE == CM_UNIQUE || MODE == CM_UNIQUE_PRED;
     static_assert(ITEMS < 32 && C >= (int)TILE, "selection mask; a tile's elements fit the ring");
+    static_assert(SM::bytes(C) <= PIPE_SMEM, "the launch's shared memory");
     extern __shared__ __align__(16) unsigned char pipe_smem[];
     constexpr int L = S % G == 0 ? S : S * G;
     __shared__ PipeBars<S, L> bars;

@@ -589,7 +589,7 @@ unsigned long long run_compact(CompactSpec& c) {
         const int items = 80 / (int)es, stages = 3;  // (CpipeShape)
         const size_t tile = (size_t)256 * items, tiles = (n + tile - 1) / tile;
         const size_t stage = tile * es + 16;
-        const size_t ring = ((220 * 1024 - stages * stage) / es - tile) / 16 * 16;
+        const size_t ring = ((trtc::PIPE_SMEM - stages * stage) / es - tile) / 16 * 16;
         ViewBuf st;
         trtc::LookbackState lst;
         if (!lookback_param(tiles, 4, st, &lst)) return kFail;
@@ -821,9 +821,10 @@ static bool reduce_by_key_pipe(const DVVectorLike& key_in, const DVVectorLike& v
     const size_t tile = (size_t)256 * items;
     const size_t halo = (ks == 1 || ks == 2 || ks == 4 || ks == 8) ? 16 / ks : 1;
     const size_t stage = round_up((tile + 2 * halo) * ks, 16) + round_up(tile * value_in.elem_size(), 16);
-    const size_t result = std::max(ks, tl.size) <= 4 ? 8 : 16;  // at most (RbkResult)
+    // a staged key and value (RbkResult) take at most: 4 + 4 bytes or odd sizes of up to 8 together 8, else 16
+    const size_t result = ks + vs <= 8 || std::max(ks, tl.size) <= 4 ? 8 : 16;
     // the rest of an SM's shared memory holds staged results (at least a tile's twice over)
-    const size_t smem = 220 * 1024;
+    const size_t smem = trtc::PIPE_SMEM;
     const size_t ring = ((smem - stages * stage) / result - tile) / 16 * 16;
     const size_t tiles = (n + tile - 1) / tile;
     uint32_t e8 = 0;
