@@ -121,16 +121,20 @@ __global__ void __launch_bounds__(256) seg_queue_kernel(const OFF* __restrict__ 
 struct SegPlan {
     uint32_t shift;   // the passes sort the codes' bits shift .. shift + 8 passes - 1
     uint32_t passes;
+    bool copies;      // the ties left are copies of one another, most likely
 };
 
 template <class K> constexpr uint32_t seg_min_passes() {
     return is_same<K, float>::value || is_same<K, double>::value ? 3u : 2u;
 }
 
-// longest run of tied keys finished in place; a longer one that is out of order sends the
-// segment to the passes over all its varying bits (any order the short form leaves keeps equal
-// keys in input order, so they start from there)
-enum { SEG_RUN = 16, SEG_FIXED = 1, SEG_LONG = 2 };
+// Work spent on a run of tied keys, in keys read and moved; a run of 16 in the worst order takes the
+// 136.  A run that needs more and is out of order sends the segment to the passes over all its
+// varying bits (any order the short form leaves keeps equal keys in input order, so they start
+// from there).
+enum { SEG_STEPS = 136, SEG_STEPS_FAR = 512, SEG_FIXED = 1, SEG_LONG = 2, SEG_DUPS = 3 };
+
+template <class K> constexpr uint32_t seg_dups3() { return seg_min_passes<K>() == 3u ? 128u : ~0u; }
 
 // the key's ordered code, descending order folded in
 template <class K, bool DESC>
@@ -158,28 +162,31 @@ TRTC_FORCEINLINE U seg_warp_or(U x) {
 }
 
 // true when two of the warp's sampled codes (`in` lanes) agree above `shift` and differ below:
-// 1 in 130 samples of 32 uniform keys at 16 bits, nearly every one of clustered keys
+// 1 in 130 samples of 32 uniform keys at 16 bits, nearly every one of clustered keys.  With `dups`
+// also when SEG_DUPS of them are copies of others: keys with so many copies (fewer than 170
+// equally likely values, or a few popular ones) leave long runs at any shift.
 template <class U>
-__device__ inline bool seg_sample_ties(U code, bool in, uint32_t shift) {
-    bool tie = false;
+__device__ inline bool seg_sample_ties(U code, bool in, uint32_t shift, bool dups) {
+    bool tie = false, copy = false;
     const uint32_t m = __ballot_sync(0xffffffffu, in);
     if (in) {
         const uint32_t peers = __match_any_sync(m, code >> shift);
         const U first = __shfl_sync(m, code, (int)__ffs(peers) - 1);
         tie = first != code;
+        copy = !tie && (peers & lanemask_lt()) != 0u;
     }
-    return __any_sync(0xffffffffu, tie);
+    return __any_sync(0xffffffffu, tie) || (dups && __popc(__ballot_sync(0xffffffffu, copy)) >= (int)SEG_DUPS);
 }
 
 // all varying bits: `diff` has a bit set where two keys of the segment differ
 template <class U>
 TRTC_FORCEINLINE SegPlan seg_full_plan(U diff) {
     const uint32_t bits = diff ? 64u - (uint32_t)__clzll((long long)(unsigned long long)diff) : 1u;
-    return {0u, (bits + 7u) / 8u};
+    return {0u, (bits + 7u) / 8u, false};
 }
 
 // the short form of at least `q0` passes where it saves one, leaves less than one tied key in
-// four for uniform keys and `ties(shift)` does not show clustered ones; else all varying bits.
+// four for uniform keys and `ties(shift, dups)` does not show clustered ones; else all varying bits.
 // q0 is 2 on chip, 3 in global memory, where a tie costs several round trips (2^24 u32 keys in
 // segments of 10,000: 891 us with two passes, 694 with three, 722 with all four), and 3 for
 // floats: sign, exponent and 7 bits of the mantissa tie most keys of a few hundred (2^24 normal
@@ -188,31 +195,41 @@ TRTC_FORCEINLINE SegPlan seg_full_plan(U diff) {
 // 250 570 -> 363, 500 438 -> 289, 2000 500 -> 412; i64 3659 -> 1263, 1388 -> 529, 1067 -> 397,
 // 1072 -> 573; f32 2054 -> 1789, 757 -> 649, 585 -> 499, 548 -> 538.  What bounds it is the
 // instruction rate of the ranking (eight ballots and an atomic per key and pass).
+// Many copies (SEG_DUPS) of more than `dups2` keys take no two-pass form: one other key in a long run
+// costs all passes again, which eight more bits make rare; more than `dups3` keys take no three-pass
+// form either (floats on chip, of which 24 bits tell too few apart; in global memory the largest).
+// B200, 2^24 keys in segments of 1000 / 2000, us, digit passes only, then the short form for every
+// segment, then this rule: u32 of 64 values 516 / 483, 659 / 623, 483 / 482; u32 ids of a Zipf(1.1)
+// popularity 518 / 485, 578 / 569, 504 / 510; f32 of 64 values 597 / 546, 925 / 842, 635 / 607; i64 ids
+// 1122 / 1053, 844 / 932, 646 / 704; of 80,000 i64 ids 2113, 4592, 2184.
 template <class U, class TIES>
-__device__ inline SegPlan seg_plan(U diff, uint32_t len, uint32_t q0, TIES ties) {
+__device__ inline SegPlan seg_plan(U diff, uint32_t len, uint32_t q0, uint32_t dups3, TIES ties) {
+    const uint32_t dups2 = 128u;
     const uint32_t bits = diff ? 64u - (uint32_t)__clzll((long long)(unsigned long long)diff) : 1u;
     for (uint32_t q = q0; q <= 3; q++)
-        if (8u * q < bits && len <= (1u << (8u * q - 2u)) && !ties(bits - 8u * q)) return {bits - 8u * q, q};
+        if (8u * q < bits && len <= (1u << (8u * q - 2u)) && !ties(bits - 8u * q, len > (q < 3u ? dups2 : dups3)))
+            return {bits - 8u * q, q, q > q0};
     return seg_full_plan(diff);
 }
 
 // Element e of a segment that is sorted by its bits from `shift` up: if it is the first of a
-// run of tied keys, insertion-sorts the run's first SEG_RUN keys.  The tied bits of a slot do
+// run of tied keys, insertion-sorts the run as far as `budget` steps go.  The tied bits of a slot do
 // not change while other threads sort their runs, so the neighbours may be read meanwhile.
 template <class K, class V, bool DESC>
 __device__ inline uint32_t seg_fix_run(volatile typename RadixKey<K>::B* sk, V* sv, uint32_t e, uint32_t len,
-                                       uint32_t shift) {
+                                       uint32_t shift, uint32_t budget) {
     typedef typename RadixKey<K>::B KB;
     typedef typename RadixKey<K>::U U;
     if (e + 1 >= len) return 0u;
     const U pre = seg_code<K, DESC>(sk[e]) >> shift;
     if ((seg_code<K, DESC>(sk[e + 1]) >> shift) != pre) return 0u;
     if (e > 0 && (seg_code<K, DESC>(sk[e - 1]) >> shift) == pre) return 0u;
+    uint32_t steps = 0;
     for (uint32_t j = e + 1; j < len; j++) {
         const KB kj = sk[j];
         const U cj = seg_code<K, DESC>(kj);
         if ((cj >> shift) != pre) break;
-        if (j - e >= (uint32_t)SEG_RUN) return (uint32_t)SEG_FIXED | (uint32_t)SEG_LONG;
+        if (++steps > budget) return (uint32_t)SEG_FIXED | (uint32_t)SEG_LONG;
         uint32_t i = j;
         if (seg_code<K, DESC>(sk[i - 1]) <= cj) continue;
         const V vj = sv[j];
@@ -220,6 +237,7 @@ __device__ inline uint32_t seg_fix_run(volatile typename RadixKey<K>::B* sk, V* 
             sk[i] = sk[i - 1];
             sv[i] = sv[i - 1];
             i--;
+            steps++;
         } while (i > e && seg_code<K, DESC>(sk[i - 1]) > cj);
         sk[i] = kj;
         sv[i] = vj;
@@ -227,29 +245,43 @@ __device__ inline uint32_t seg_fix_run(volatile typename RadixKey<K>::B* sk, V* 
     return (uint32_t)SEG_FIXED;
 }
 
-// seg_fix_run for the elements first, first + stride, ... below end: the ties are collected
-// for 32 of them before the first run is sorted, so the lanes of a warp sort their runs at the
-// same time (row by row nearly every row of 32 has one lane with a run)
-template <class K, class V, bool DESC>
-__device__ inline uint32_t seg_fix_runs(typename RadixKey<K>::B* sk, V* sv, uint32_t first, uint32_t stride,
-                                        uint32_t end, uint32_t len, uint32_t shift) {
+// Bit r: element e = first + r * stride (below end, at most 32 of them) ties with the next one.  The ties
+// are collected before the first run is sorted, so the lanes of a warp sort their runs at the same
+// time (row by row nearly every row of 32 has one lane with a run).
+// INV: also whether any of these ties is out of order (copies are not).
+template <class K, bool DESC, bool INV>
+__device__ inline uint32_t seg_tie_mask(const typename RadixKey<K>::B* sk, uint32_t first, uint32_t stride,
+                                        uint32_t end, uint32_t len, uint32_t shift, bool& inverted) {
+    typedef typename RadixKey<K>::U U;
     const uint32_t last = min(end, len - 1u);  // the segment's last key starts no run
-    uint32_t fixed = 0;
-    for (; first < last; first += 32u * stride) {
-        uint32_t mask = 0;
+    uint32_t mask = 0;
 #pragma unroll 4
-        for (uint32_t r = 0; r < 32u; r++) {
-            const uint32_t e = first + r * stride;
-            if (e >= last) break;
-            const bool tie = ((seg_code<K, DESC>(sk[e]) ^ seg_code<K, DESC>(sk[e + 1])) >> shift) == 0;
-            mask |= tie ? 1u << r : 0u;
-        }
-        while (mask) {
-            const uint32_t e = first + (uint32_t)(__ffs((int)mask) - 1) * stride;
-            mask &= mask - 1u;
-            fixed |= seg_fix_run<K, V, DESC>(sk, sv, e, len, shift);
-        }
+    for (uint32_t r = 0; r < 32u; r++) {
+        const uint32_t e = first + r * stride;
+        if (e >= last) break;
+        const U a = seg_code<K, DESC>(sk[e]), b = seg_code<K, DESC>(sk[e + 1]);
+        const bool tie = ((a ^ b) >> shift) == 0;
+        mask |= tie ? 1u << r : 0u;
+        if constexpr (INV) inverted |= tie && a > b;
     }
+    return mask;
+}
+// the same for the ties of a mask (asked where a plan expects copies and the answer takes a barrier)
+template <class K, bool DESC>
+__device__ inline bool seg_mask_inverted(const typename RadixKey<K>::B* sk, uint32_t first, uint32_t stride, uint32_t mask) {
+    bool inv = false;
+    for (; mask; mask &= mask - 1u) {
+        const uint32_t e = first + (uint32_t)(__ffs((int)mask) - 1) * stride;
+        inv |= seg_code<K, DESC>(sk[e]) > seg_code<K, DESC>(sk[e + 1]);
+    }
+    return inv;
+}
+template <class K, class V, bool DESC>
+__device__ inline uint32_t seg_fix_mask(typename RadixKey<K>::B* sk, V* sv, uint32_t first, uint32_t stride,
+                                        uint32_t mask, uint32_t len, uint32_t shift) {
+    uint32_t fixed = 0;
+    for (; mask; mask &= mask - 1u)
+        fixed |= seg_fix_run<K, V, DESC>(sk, sv, first + (uint32_t)(__ffs((int)mask) - 1) * stride, len, shift, SEG_STEPS);
     return fixed;
 }
 
@@ -379,8 +411,8 @@ __device__ inline void seg_warp_sort_scan(const typename RadixKey<K>::B* ik, con
     for (int i = 0; i < ITEMS; i++)
         if (i < IT && (uint32_t)i * 32u + lane < len) diff |= seg_code<K, DESC>(k[i]) ^ ref;
     diff = seg_warp_or(diff);
-    SegPlan plan = seg_plan(diff, len, Q0, [&](uint32_t sh) {
-        return seg_sample_ties(seg_code<K, DESC>(k[0]), lane < len, sh);
+    SegPlan plan = seg_plan(diff, len, Q0, seg_dups3<K>(), [&](uint32_t sh, bool dups) {
+        return seg_sample_ties(seg_code<K, DESC>(k[0]), lane < len, sh, dups);
     });
     uint32_t shift = plan.shift;
     for (uint32_t p = 0; p < plan.passes; p++) {
@@ -441,8 +473,11 @@ __device__ inline void seg_warp_sort_scan(const typename RadixKey<K>::B* ik, con
         shift += 8u;
         if (p + 1 < plan.passes || plan.shift == 0) continue;
         // the last pass of the short form: the runs of tied keys
+        bool inverted = false;
+        const uint32_t mask = seg_tie_mask<K, DESC, true>(sk, lane, 32u, len, len, plan.shift, inverted);
+        if (!__any_sync(0xffffffffu, inverted)) continue;
         const uint32_t fixed =
-            __reduce_or_sync(0xffffffffu, seg_fix_runs<K, V, DESC>(sk, sv, lane, 32u, len, len, plan.shift));
+            __reduce_or_sync(0xffffffffu, seg_fix_mask<K, V, DESC>(sk, sv, lane, 32u, mask, len, plan.shift));
         __syncwarp();
         if (fixed) {
 #pragma unroll
@@ -546,10 +581,10 @@ __device__ __noinline__ void seg_group_sort_scan(const typename RadixKey<K>::B* 
         diff |= (U)(((unsigned long long)cw[1] << 32) | cw[0]);
     }
     // (every warp looks at the same G samples, spread over the segment)
-    SegPlan plan = seg_plan(diff, len, Q0, [&](uint32_t sh) {
+    SegPlan plan = seg_plan(diff, len, Q0, seg_dups3<K>(), [&](uint32_t sh, bool dups) {
         bool tie = false;
         for (uint32_t w = 0; w < G; w++)
-            tie |= seg_sample_ties(seg_code<K, DESC>(ik[(len / GT) * (w * 32u + lane)]), true, sh);
+            tie |= seg_sample_ties(seg_code<K, DESC>(ik[(len / GT) * (w * 32u + lane)]), true, sh, dups);
         return tie;
     });
     gsync();  // the counters are free
@@ -615,8 +650,19 @@ __device__ __noinline__ void seg_group_sort_scan(const typename RadixKey<K>::B* 
         if (p + 1 == plan.passes) {
             if (plan.shift == 0) break;
             // the last pass of the short form: the runs of tied keys
+            bool out = false;
+            const uint32_t mask = seg_tie_mask<K, DESC, false>(sk, wbase + lane, 32u, wbase + wn, len, plan.shift, out);
+            if (plan.copies) {
+                out = __any_sync(0xffffffffu, seg_mask_inverted<K, DESC>(sk, wbase + lane, 32u, mask));
+                if (lane == 0) wh[0] = out ? 1u : 0u;
+                gsync();
+                uint32_t any = 0;
+                for (uint32_t w = 0; w < G; w++) any |= s_whist[(gw0 + w) * 256];
+                gsync();  // the counters are free
+                if (!any) break;
+            }
             uint32_t fixed = __reduce_or_sync(
-                0xffffffffu, seg_fix_runs<K, V, DESC>(sk, va, wbase + lane, 32u, wbase + wn, len, plan.shift));
+                0xffffffffu, seg_fix_mask<K, V, DESC>(sk, va, wbase + lane, 32u, mask, len, plan.shift));
             if (lane == 0) s_wsum[warp] = fixed;
             gsync();  // the runs are sorted
             fixed = 0;
@@ -810,17 +856,64 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
             return x;
         };
         // eight samples spread over n >= 256 keys; two ties among uniform keys are 1 in 600
-        auto sampled = [&](const KB* k, uint32_t n, uint32_t sh) -> bool {
-            const bool tie = seg_sample_ties(seg_code<K, DESC>(k[(n >> 8) * threadIdx.x]), true, sh);
+        auto sampled = [&](const KB* k, uint32_t n, uint32_t sh, bool dups) -> bool {
+            const bool tie = seg_sample_ties(seg_code<K, DESC>(k[(n >> 8) * threadIdx.x]), true, sh, dups);
             return __syncthreads_count(tie && lane == 0) >= 2;
         };
-        // finishes the runs of tied keys that a short form left; false: some run is too long
-        auto sorted_runs = [&](KB* k, V* v, uint32_t n, uint32_t shift) -> bool {
-            const uint32_t fixed = seg_fix_runs<K, V, DESC>(k, v, threadIdx.x, 256u, n, n, shift);
-            if (!__syncthreads_or((int)(fixed & (uint32_t)SEG_LONG))) return true;
+        // finishes the runs of tied keys that a short form left; false: some run takes too long
+        auto sorted = [&](const KB* k, uint32_t n) -> bool {
             bool inv = false;
             for (uint32_t e = threadIdx.x; e < n; e += 256) inv |= seg_inverted<K, DESC>(k, e);
             return !__syncthreads_or(inv);
+        };
+        auto fix_on_chip = [&](uint32_t n, const SegPlan& plan) -> bool {
+            bool inv = false;
+            const uint32_t mask = seg_tie_mask<K, DESC, false>(s_k, threadIdx.x, 256u, n, n, plan.shift, inv);
+            if (plan.copies && !__syncthreads_or(seg_mask_inverted<K, DESC>(s_k, threadIdx.x, 256u, mask))) return true;
+            const uint32_t fixed = seg_fix_mask<K, V, DESC>(s_k, s_v, threadIdx.x, 256u, mask, n, plan.shift);
+            if (!__syncthreads_or((int)(fixed & (uint32_t)SEG_LONG))) return true;
+            return sorted(s_k, n);
+        };
+        // the same in global memory, where looking into every run of ties can cost more than the passes
+        // saved: the first inverted tie of a run (walking back finds none before it) lists the run's
+        // first key, in the digit counters, which every pass clears first
+        auto fix_in_memory = [&](KB* k, V* v, uint32_t n, uint32_t shift) -> bool {
+            if (threadIdx.x == 0) s_whist[0] = 0;
+            __syncthreads();
+            bool inv = false, far = false;
+            for (uint32_t e = threadIdx.x; e + 1 < n; e += 256) {
+                const U a = seg_code<K, DESC>(k[e]), b = seg_code<K, DESC>(k[e + 1]);
+                if (((a ^ b) >> shift) != 0 || a <= b) continue;
+                inv = true;
+                uint32_t st = e;
+                U next = a;
+                bool lead = true;
+                while (lead && st > 0) {
+                    const U c = seg_code<K, DESC>(k[st - 1]);
+                    if (((c ^ a) >> shift) != 0) break;
+                    if (e - st >= (uint32_t)SEG_STEPS_FAR) far = true;
+                    lead = c <= next && !far;
+                    next = c;
+                    st--;
+                }
+                if (!lead) continue;
+                const uint32_t at = atomicAdd(&s_whist[0], 1u);
+                if (at < 2047u) s_whist[1u + at] = st;
+            }
+            if (!__syncthreads_or(inv)) return true;
+            const uint32_t runs = s_whist[0];
+            if (__syncthreads_or(far) == 0 && runs <= 2047u) {
+                uint32_t fixed = 0;
+                for (uint32_t i = threadIdx.x; i < runs; i += 256)
+                    fixed |= seg_fix_run<K, V, DESC>(k, v, s_whist[1u + i], n, shift, SEG_STEPS_FAR);
+                if (!__syncthreads_or((int)(fixed & (uint32_t)SEG_LONG))) return true;
+            } else if (runs > 2047u) {
+                uint32_t fixed = 0;
+                for (uint32_t e = threadIdx.x; e < n; e += 8192u)
+                    fixed |= seg_fix_mask<K, V, DESC>(k, v, e, 256u, seg_tie_mask<K, DESC, false>(k, e, 256u, n, n, shift, inv), n, shift);
+                if (!__syncthreads_or((int)(fixed & (uint32_t)SEG_LONG))) return true;
+            }
+            return sorted(k, n);
         };
         // one stable pass by the digit at `shift` through global memory; s_run: the digits' starts
         auto scatter = [&](const KB* sk, const V* sv, KB* dk, V* dv, uint32_t shift) {
@@ -864,9 +957,11 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
             KB* dk = tk + base;
             V* dv = tv + base;
             const U ref = seg_code<K, DESC>(gk[0]);
-            // from two CTA tiles up (16 keys a thread: 8192 keys; 2^24 u32 keys in segments of
-            // 40,000: 829 us by LSD passes, 598 this way, one segment of 100,000 951 and 667; one of
-            // 5000 79 and 96):
+            // from two CTA tiles up, four of floats (16 keys a thread: 8192 and 16,384 keys; 2^24 u32 keys in
+            // segments of 40,000: 829 us by LSD passes, 598 this way, one segment of 100,000 951 and 667; of
+            // 9000 717 and 678; f32 of 14,000 824 and 858; i64 of 9000 1757 and 1102).  4-byte keys of 2.5 to
+            // 3 tiles, where LSD passes run over full tiles and there would be twice the buckets, half as
+            // full: u32 of 12,000 655 and 719, one of them 133 and 149, one of 10,291 123 and 144.
             // one pass by the top bits of those that vary puts the keys into buckets of 5/8 of a
             // warp's share on average (up to 256 of them); each is then sorted on chip.  Which bits
             // vary is read off a sample of 256 keys and checked by the pass that counts them all.
@@ -880,10 +975,16 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
             __syncthreads();
             atomicAdd(&s_hist[0][seg_digit<K, DESC>(sample, top)], 1u);
             __syncthreads();
-            // (clustered keys, the exponents of floats, fill a bucket: seen in the sample already)
+            // (clustered keys, the exponents of floats, fill a bucket: seen in the sample already.)  With
+            // many copies a bucket that is too large is certain sooner, and 4-byte keys take the LSD
+            // passes (u32 ids of a Zipf popularity in segments of 10,000: 702 us, in buckets 1098)
             const uint32_t seen = s_hist[0][threadIdx.x];
-            bool one = __syncthreads_or(len <= 2u * (uint32_t)TILE ||
-                                        (seen >= 16u && (unsigned long long)seen * (len >> 8) > 2ull * TILE));
+            const bool copies = __syncthreads_count(seg_sample_ties(seg_code<K, DESC>(sample), true, 0u, true) && lane == 0) >= 2;
+            const bool few = seg_min_passes<K>() == 3u ? len <= 4u * (uint32_t)TILE
+                                                       : len <= 2u * (uint32_t)TILE ||
+                                                             (sizeof(U) == 4 && len > 5u * (uint32_t)TILE / 2u && len <= 3u * (uint32_t)TILE);
+            bool one = __syncthreads_or(few || (sizeof(U) == 4 && copies) ||
+                                        (seen >= 16u && (unsigned long long)seen * (len >> 8) > (copies ? 1ull : 2ull) * TILE));
             if (!one) {
                 s_hist[0][threadIdx.x] = 0;
                 __syncthreads();
@@ -959,7 +1060,7 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
 #pragma unroll 4
                     for (uint32_t e = threadIdx.x; e < len; e += 256) diff |= seg_code<K, DESC>(gk[e]) ^ ref;
                     diff = block_or(diff);
-                    plan = seg_plan(diff, len, 3u, [&](uint32_t sh) { return sampled(gk, len, sh); });
+                    plan = seg_plan(diff, len, 3u, 1u << 16, [&](uint32_t sh, bool dups) { return sampled(gk, len, sh, dups); });
                 } else {  // (finding the varying bits, three passes and the ties cost as much as four passes)
                     diff = ~U(0);
                     plan = seg_full_plan(diff);
@@ -988,7 +1089,7 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
                         KB* t1 = sk; sk = dk; dk = t1;
                         V* t2 = sv; sv = dv; dv = t2;
                     }
-                    if (plan.shift == 0 || sorted_runs(sk, sv, len, plan.shift)) break;
+                    if (plan.shift == 0 || fix_in_memory(sk, sv, len, plan.shift)) break;
                     plan = seg_full_plan(diff);
                 }
                 // the sorted segment is in sk/sv (the caller's arrays after an even number of passes);
@@ -1035,8 +1136,8 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
             for (int i = 0; i < ITEMS; i++)
                 if (i < IT && wbase + (uint32_t)i * 32u + lane < n) diff |= seg_code<K, DESC>(k[i]) ^ ref;
             diff = block_or(diff);
-            SegPlan plan = seg_plan(diff, n, seg_min_passes<K>(),
-                                    [&](uint32_t sh) { return sampled(ik, n, sh); });
+            SegPlan plan = seg_plan(diff, n, seg_min_passes<K>(), seg_dups3<K>(),
+                                    [&](uint32_t sh, bool dups) { return sampled(ik, n, sh, dups); });
             uint32_t shift = plan.shift;
             for (uint32_t p = 0; p < plan.passes; p++) {
                 seg_rank_tile<K, DESC, ITEMS>(k, pos, IT, n, shift, s_whist, s_cnt, s_start, s_wsum);
@@ -1048,7 +1149,7 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
                 __syncthreads();
                 shift += 8u;
                 if (p + 1 == plan.passes) {
-                    if (plan.shift == 0 || sorted_runs(s_k, s_v, n, plan.shift)) break;
+                    if (plan.shift == 0 || fix_on_chip(n, plan)) break;
                     plan = seg_full_plan(diff);
                     shift = 0;
                     p = ~0u;  // from the first pass again
