@@ -346,6 +346,13 @@ TRTC_FORCEINLINE uint32_t radix_digit_sel(typename RadixKey<K>::B k, uint32_t se
     return DESC ? (d ^ 0xFFu) : d;
 }
 
+// Do the digit passes run as resident CTAs that take tile after tile?  Not of float keys: their passes are
+// bound by the instruction rate (three key codes per key and pass), and as a loop they lose more than
+// launches cost.  B200, us per sort, a CTA per tile against resident CTAs: 2^28 float keys 4646 / 4772,
+// descending 4655 / 4960, pairs 5623 / 5901; 30 M 592 / 602, pairs 709 / 733; 2^20 87 / 89, pairs 95 / 98.
+// (Doubles: 2^28 keys 15,623 / 15,071, pairs 18,122 / 17,546; u32 keys 4.54 / 4.36 ms, pairs 5.67 / 5.56.)
+template <class K> struct RadixResident { static constexpr bool value = !is_same<K, float>::value; };
+
 template <bool B> struct BoolC { static constexpr bool value = B; };
 
 #ifndef TRTC_RADIX_MINB  // resident CTAs per SM the pass kernel is compiled for
@@ -502,7 +509,7 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     // resident CTAs 5.55 and 0.398 ms, 2 us).  Keys-only passes draw the next ticket before they
     // write a tile out (2^28 keys 4.49 -> 4.35 ms); pairs, which write twice as much meanwhile and
     // so hold back the tiles that wait for theirs, after it (5.55 ms; before it 5.90 ms).
-    constexpr bool EARLY = !HAS_VALS;
+    constexpr bool EARLY = !HAS_VALS && RadixResident<K>::value;
     const size_t tiles = (n + TILE - 1) / TILE;
     uint32_t vphase = 0;
     if (VB && threadIdx.x == 0) mbar_init_one(&s_vbar);
@@ -736,7 +743,7 @@ __global__ void __launch_bounds__(BLOCK, TRTC_RADIX_MINB(ITEMS)) radix_pass_kern
     };
     if (full) write_tile(BoolC<true>());
     else write_tile(BoolC<false>());
-    if (gridDim.x >= tiles) return;  // a tile per CTA
+    if (!RadixResident<K>::value || gridDim.x >= tiles) return;  // a tile per CTA
     vphase ^= vbulk ? 1u : 0u;
     if (EARLY && threadIdx.x == 0) s_tile = next;
     // this tile's ordinary stores to s_vals come before the next tile's bulk copy into it (another

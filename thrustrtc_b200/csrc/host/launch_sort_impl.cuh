@@ -140,7 +140,7 @@ static bool radix_sort_run(K* keys, V* vals0, size_t n, cudaStream_t s, int vals
             int v = 0;
             return TRTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, pass_kernel, BLOCK, smem)) && v > 0 ? v : 1;
         }();
-        const size_t pgrid = (size_t)per_sm * sms < tiles ? (size_t)per_sm * sms : tiles;
+        const size_t pgrid = RadixResident<K>::value && (size_t)per_sm * sms < tiles ? (size_t)per_sm * sms : tiles;
         for (int p = 0; p < D; p++) {
             launch_dependent(pass_kernel, (unsigned)pgrid, BLOCK, smem, s, bufs, n, ctrl, p, (ST*)st0, (ST*)st1,
                              vals_from_index, pf);

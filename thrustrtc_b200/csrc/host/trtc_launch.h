@@ -12,7 +12,8 @@ enum : int { COMPACT_NOT_EQUAL = 2, COMPACT_UNIQUE = 5 };
 // CTAs per SM of the reduce kernel: 4 x 256 threads with 16 loads each cover the memory latency, and
 // the last CTA folds half as many partials as with 8 (B200, per launch, float sums of 2^28 / 67 M /
 // 16.8 M / 4 M: 2 CTAs 191 / 56 / 21.8 / 12.1 us, 3: 166 / 50 / 20.7 / 11.9, 4: 160 / 48 / 20.7 / 11.8,
-// 8: 167 / 51 / 23.4 / 14.4)
+// 8: 167 / 51 / 23.4 / 14.4.  Per call with L2 flushed before each, 2^28 / 2^27 / 2^26 / 16.8 M floats:
+// 4: 195 / 121 / 76 / 36 us, 8: 197 / 117 / 74 / 39)
 enum : int { REDUCE_CTAS = 4 };
 
 // compactions of fewer elements keep the two-phase kernel, whose one tile per CTA is done before the
