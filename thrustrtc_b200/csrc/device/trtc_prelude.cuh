@@ -125,7 +125,9 @@ TRTC_FORCEINLINE void prefetch_l2_range(const E* base, size_t first, size_t coun
 TRTC_FORCEINLINE bool spin_continue(uint32_t& spins, const uint32_t* err) {
     ++spins;
     if (spins > TRTC_SPIN_LIMIT) return false;
-    if ((spins & 255u) == 0 && err && *(volatile const uint32_t*)err) return false;
+    // the error word lies in host memory: read seldom, or the reads of many waiting warps hold up those
+    // that everybody waits for
+    if ((spins & 4095u) == 0 && err && *(volatile const uint32_t*)err) return false;
     backoff(spins);
     return true;
 }
