@@ -121,20 +121,21 @@ __global__ void __launch_bounds__(256) seg_queue_kernel(const OFF* __restrict__ 
 struct SegPlan {
     uint32_t shift;   // the passes sort the codes' bits shift .. shift + 8 passes - 1
     uint32_t passes;
-    bool copies;      // the ties left are copies of one another, most likely
+    // of a form that may take two passes: the ties left by three are copies of one another, most likely
+    TRTC_FORCEINLINE bool copies(uint32_t q0) const { return q0 == 2u && passes == 3u; }
 };
 
 template <class K> constexpr uint32_t seg_min_passes() {
     return is_same<K, float>::value || is_same<K, double>::value ? 3u : 2u;
 }
 
-// Work spent on a run of tied keys, in keys read and moved; a run of 16 in the worst order takes the
-// 136.  A run that needs more and is out of order sends the segment to the passes over all its
+// Longest run of tied keys finished in place on chip, and the work spent on one in global memory, in keys
+// read and moved.  A longer one that is out of order sends the segment to the passes over all its
 // varying bits (any order the short form leaves keeps equal keys in input order, so they start
 // from there).
-enum { SEG_STEPS = 136, SEG_STEPS_FAR = 512, SEG_FIXED = 1, SEG_LONG = 2, SEG_DUPS = 3 };
+enum { SEG_RUN = 16, SEG_STEPS_FAR = 512, SEG_FIXED = 1, SEG_LONG = 2, SEG_DUPS = 3 };
 
-template <class K> constexpr uint32_t seg_dups3() { return seg_min_passes<K>() == 3u ? 128u : ~0u; }
+template <class K> constexpr uint32_t seg_dups3() { return sizeof(typename RadixKey<K>::U) == 4 ? 128u : ~0u; }
 
 // the key's ordered code, descending order folded in
 template <class K, bool DESC>
@@ -182,7 +183,7 @@ __device__ inline bool seg_sample_ties(U code, bool in, uint32_t shift, bool dup
 template <class U>
 TRTC_FORCEINLINE SegPlan seg_full_plan(U diff) {
     const uint32_t bits = diff ? 64u - (uint32_t)__clzll((long long)(unsigned long long)diff) : 1u;
-    return {0u, (bits + 7u) / 8u, false};
+    return {0u, (bits + 7u) / 8u};
 }
 
 // the short form of at least `q0` passes where it saves one, leaves less than one tied key in
@@ -195,29 +196,30 @@ TRTC_FORCEINLINE SegPlan seg_full_plan(U diff) {
 // 250 570 -> 363, 500 438 -> 289, 2000 500 -> 412; i64 3659 -> 1263, 1388 -> 529, 1067 -> 397,
 // 1072 -> 573; f32 2054 -> 1789, 757 -> 649, 585 -> 499, 548 -> 538.  What bounds it is the
 // instruction rate of the ranking (eight ballots and an atomic per key and pass).
-// Many copies (SEG_DUPS) of more than `dups2` keys take no two-pass form: one other key in a long run
-// costs all passes again, which eight more bits make rare; more than `dups3` keys take no three-pass
-// form either (floats on chip, of which 24 bits tell too few apart; in global memory the largest).
-// B200, 2^24 keys in segments of 1000 / 2000, us, digit passes only, then the short form for every
-// segment, then this rule: u32 of 64 values 516 / 483, 659 / 623, 483 / 482; u32 ids of a Zipf(1.1)
-// popularity 518 / 485, 578 / 569, 504 / 510; f32 of 64 values 597 / 546, 925 / 842, 635 / 607; i64 ids
-// 1122 / 1053, 844 / 932, 646 / 704; of 80,000 i64 ids 2113, 4592, 2184.
+// Segments of more than 128 keys of which many are copies (SEG_DUPS) take no two-pass form: one other key
+// in a long run of copies costs all passes again, which eight more bits make rare.  4-byte keys take all
+// digits then (`dups3`): the question whether the runs are in order costs their kernel 2 to 3 % where there
+// are none, more than a pass saved in segments of copies is worth.  B200, 2^24 keys in segments of 250 / 1000 /
+// 2000, us, all digits by the former passes, the short form for every segment, this rule: u32 of 64 values
+// 555 / 516 / 483, 526 / 659 / 623, 524 / 545 / 543; u32 ids of a Zipf(1.1) popularity 558 / 518 / 485, 504 / 578 /
+// 569, 531 / 545 / 545; f32 of 64 values 761 / 597 / 546, 865 / 925 / 842, 728 / 635 / 605; i64 of 64 values 1362 /
+// 1117 / 1046, 759 / 942 / 901, 627 / 608 / 631; i64 ids in segments of 80,000 2113, 4592, 2184.
 template <class U, class TIES>
 __device__ inline SegPlan seg_plan(U diff, uint32_t len, uint32_t q0, uint32_t dups3, TIES ties) {
     const uint32_t dups2 = 128u;
     const uint32_t bits = diff ? 64u - (uint32_t)__clzll((long long)(unsigned long long)diff) : 1u;
     for (uint32_t q = q0; q <= 3; q++)
         if (8u * q < bits && len <= (1u << (8u * q - 2u)) && !ties(bits - 8u * q, len > (q < 3u ? dups2 : dups3)))
-            return {bits - 8u * q, q, q > q0};
+            return {bits - 8u * q, q};
     return seg_full_plan(diff);
 }
 
 // Element e of a segment that is sorted by its bits from `shift` up: if it is the first of a
-// run of tied keys, insertion-sorts the run as far as `budget` steps go.  The tied bits of a slot do
+// run of tied keys, insertion-sorts the run's first SEG_RUN keys, or as far as SEG_STEPS_FAR go (FAR).  The tied bits of a slot do
 // not change while other threads sort their runs, so the neighbours may be read meanwhile.
-template <class K, class V, bool DESC>
+template <class K, class V, bool DESC, bool FAR>
 __device__ inline uint32_t seg_fix_run(volatile typename RadixKey<K>::B* sk, V* sv, uint32_t e, uint32_t len,
-                                       uint32_t shift, uint32_t budget) {
+                                       uint32_t shift) {
     typedef typename RadixKey<K>::B KB;
     typedef typename RadixKey<K>::U U;
     if (e + 1 >= len) return 0u;
@@ -229,7 +231,7 @@ __device__ inline uint32_t seg_fix_run(volatile typename RadixKey<K>::B* sk, V* 
         const KB kj = sk[j];
         const U cj = seg_code<K, DESC>(kj);
         if ((cj >> shift) != pre) break;
-        if (++steps > budget) return (uint32_t)SEG_FIXED | (uint32_t)SEG_LONG;
+        if (FAR ? ++steps > (uint32_t)SEG_STEPS_FAR : j - e >= (uint32_t)SEG_RUN) return (uint32_t)SEG_FIXED | (uint32_t)SEG_LONG;
         uint32_t i = j;
         if (seg_code<K, DESC>(sk[i - 1]) <= cj) continue;
         const V vj = sv[j];
@@ -237,7 +239,7 @@ __device__ inline uint32_t seg_fix_run(volatile typename RadixKey<K>::B* sk, V* 
             sk[i] = sk[i - 1];
             sv[i] = sv[i - 1];
             i--;
-            steps++;
+            if (FAR) steps++;
         } while (i > e && seg_code<K, DESC>(sk[i - 1]) > cj);
         sk[i] = kj;
         sv[i] = vj;
@@ -245,44 +247,46 @@ __device__ inline uint32_t seg_fix_run(volatile typename RadixKey<K>::B* sk, V* 
     return (uint32_t)SEG_FIXED;
 }
 
-// Bit r: element e = first + r * stride (below end, at most 32 of them) ties with the next one.  The ties
-// are collected before the first run is sorted, so the lanes of a warp sort their runs at the same
-// time (row by row nearly every row of 32 has one lane with a run).
-// INV: also whether any of these ties is out of order (copies are not).
-template <class K, bool DESC, bool INV>
-__device__ inline uint32_t seg_tie_mask(const typename RadixKey<K>::B* sk, uint32_t first, uint32_t stride,
-                                        uint32_t end, uint32_t len, uint32_t shift, bool& inverted) {
-    typedef typename RadixKey<K>::U U;
+// seg_fix_run for the elements first, first + stride, ... below end: the ties are collected
+// for 32 of them before the first run is sorted, so the lanes of a warp sort their runs at the
+// same time (row by row nearly every row of 32 has one lane with a run)
+template <class K, class V, bool DESC>
+__device__ inline uint32_t seg_fix_runs(typename RadixKey<K>::B* sk, V* sv, uint32_t first, uint32_t stride,
+                                        uint32_t end, uint32_t len, uint32_t shift) {
     const uint32_t last = min(end, len - 1u);  // the segment's last key starts no run
-    uint32_t mask = 0;
+    uint32_t fixed = 0;
+    for (; first < last; first += 32u * stride) {
+        uint32_t mask = 0;
 #pragma unroll 4
-    for (uint32_t r = 0; r < 32u; r++) {
-        const uint32_t e = first + r * stride;
-        if (e >= last) break;
-        const U a = seg_code<K, DESC>(sk[e]), b = seg_code<K, DESC>(sk[e + 1]);
-        const bool tie = ((a ^ b) >> shift) == 0;
-        mask |= tie ? 1u << r : 0u;
-        if constexpr (INV) inverted |= tie && a > b;
+        for (uint32_t r = 0; r < 32u; r++) {
+            const uint32_t e = first + r * stride;
+            if (e >= last) break;
+            const bool tie = ((seg_code<K, DESC>(sk[e]) ^ seg_code<K, DESC>(sk[e + 1])) >> shift) == 0;
+            mask |= tie ? 1u << r : 0u;
+        }
+        while (mask) {
+            const uint32_t e = first + (uint32_t)(__ffs((int)mask) - 1) * stride;
+            mask &= mask - 1u;
+            fixed |= seg_fix_run<K, V, DESC, false>(sk, sv, e, len, shift);
+        }
     }
-    return mask;
+    return fixed;
 }
-// the same for the ties of a mask (asked where a plan expects copies and the answer takes a barrier)
+
+// Is any of the ties among these elements out of order?  (Copies are not: where a plan expects them, nobody
+// looks into the runs of a segment without an inverted tie.)
 template <class K, bool DESC>
-__device__ inline bool seg_mask_inverted(const typename RadixKey<K>::B* sk, uint32_t first, uint32_t stride, uint32_t mask) {
+__device__ inline bool seg_ties_inverted(const typename RadixKey<K>::B* sk, uint32_t first, uint32_t stride, uint32_t end,
+                                         uint32_t len, uint32_t shift) {
+    typedef typename RadixKey<K>::U U;
+    const uint32_t last = min(end, len - 1u);
     bool inv = false;
-    for (; mask; mask &= mask - 1u) {
-        const uint32_t e = first + (uint32_t)(__ffs((int)mask) - 1) * stride;
-        inv |= seg_code<K, DESC>(sk[e]) > seg_code<K, DESC>(sk[e + 1]);
+#pragma unroll 4
+    for (; first < last; first += stride) {
+        const U a = seg_code<K, DESC>(sk[first]), b = seg_code<K, DESC>(sk[first + 1]);
+        inv |= ((a ^ b) >> shift) == 0 && a > b;
     }
     return inv;
-}
-template <class K, class V, bool DESC>
-__device__ inline uint32_t seg_fix_mask(typename RadixKey<K>::B* sk, V* sv, uint32_t first, uint32_t stride,
-                                        uint32_t mask, uint32_t len, uint32_t shift) {
-    uint32_t fixed = 0;
-    for (; mask; mask &= mask - 1u)
-        fixed |= seg_fix_run<K, V, DESC>(sk, sv, first + (uint32_t)(__ffs((int)mask) - 1) * stride, len, shift, SEG_STEPS);
-    return fixed;
 }
 
 // true where element e is smaller than the one before it
@@ -473,11 +477,12 @@ __device__ inline void seg_warp_sort_scan(const typename RadixKey<K>::B* ik, con
         shift += 8u;
         if (p + 1 < plan.passes || plan.shift == 0) continue;
         // the last pass of the short form: the runs of tied keys
-        bool inverted = false;
-        const uint32_t mask = seg_tie_mask<K, DESC, true>(sk, lane, 32u, len, len, plan.shift, inverted);
-        if (!__any_sync(0xffffffffu, inverted)) continue;
+        if constexpr (sizeof(U) == 8 || Q0 == 3u)
+            if ((Q0 == 3u || plan.copies(Q0)) &&
+                !__any_sync(0xffffffffu, seg_ties_inverted<K, DESC>(sk, lane, 32u, len, len, plan.shift)))
+                continue;
         const uint32_t fixed =
-            __reduce_or_sync(0xffffffffu, seg_fix_mask<K, V, DESC>(sk, sv, lane, 32u, mask, len, plan.shift));
+            __reduce_or_sync(0xffffffffu, seg_fix_runs<K, V, DESC>(sk, sv, lane, 32u, len, len, plan.shift));
         __syncwarp();
         if (fixed) {
 #pragma unroll
@@ -650,10 +655,9 @@ __device__ __noinline__ void seg_group_sort_scan(const typename RadixKey<K>::B* 
         if (p + 1 == plan.passes) {
             if (plan.shift == 0) break;
             // the last pass of the short form: the runs of tied keys
-            bool out = false;
-            const uint32_t mask = seg_tie_mask<K, DESC, false>(sk, wbase + lane, 32u, wbase + wn, len, plan.shift, out);
-            if (plan.copies) {
-                out = __any_sync(0xffffffffu, seg_mask_inverted<K, DESC>(sk, wbase + lane, 32u, mask));
+            if (sizeof(U) == 8 && plan.copies(Q0)) {
+                const bool out =
+                    __any_sync(0xffffffffu, seg_ties_inverted<K, DESC>(sk, wbase + lane, 32u, wbase + wn, len, plan.shift));
                 if (lane == 0) wh[0] = out ? 1u : 0u;
                 gsync();
                 uint32_t any = 0;
@@ -662,7 +666,7 @@ __device__ __noinline__ void seg_group_sort_scan(const typename RadixKey<K>::B* 
                 if (!any) break;
             }
             uint32_t fixed = __reduce_or_sync(
-                0xffffffffu, seg_fix_mask<K, V, DESC>(sk, va, wbase + lane, 32u, mask, len, plan.shift));
+                0xffffffffu, seg_fix_runs<K, V, DESC>(sk, va, wbase + lane, 32u, wbase + wn, len, plan.shift));
             if (lane == 0) s_wsum[warp] = fixed;
             gsync();  // the runs are sorted
             fixed = 0;
@@ -867,10 +871,10 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
             return !__syncthreads_or(inv);
         };
         auto fix_on_chip = [&](uint32_t n, const SegPlan& plan) -> bool {
-            bool inv = false;
-            const uint32_t mask = seg_tie_mask<K, DESC, false>(s_k, threadIdx.x, 256u, n, n, plan.shift, inv);
-            if (plan.copies && !__syncthreads_or(seg_mask_inverted<K, DESC>(s_k, threadIdx.x, 256u, mask))) return true;
-            const uint32_t fixed = seg_fix_mask<K, V, DESC>(s_k, s_v, threadIdx.x, 256u, mask, n, plan.shift);
+            if (sizeof(U) == 8 && plan.copies(seg_min_passes<K>()) &&
+                !__syncthreads_or(seg_ties_inverted<K, DESC>(s_k, threadIdx.x, 256u, n, n, plan.shift)))
+                return true;
+            const uint32_t fixed = seg_fix_runs<K, V, DESC>(s_k, s_v, threadIdx.x, 256u, n, n, plan.shift);
             if (!__syncthreads_or((int)(fixed & (uint32_t)SEG_LONG))) return true;
             return sorted(s_k, n);
         };
@@ -905,12 +909,11 @@ __global__ void __launch_bounds__(256, MINB) seg_sort_scan_kernel(typename Radix
             if (__syncthreads_or(far) == 0 && runs <= 2047u) {
                 uint32_t fixed = 0;
                 for (uint32_t i = threadIdx.x; i < runs; i += 256)
-                    fixed |= seg_fix_run<K, V, DESC>(k, v, s_whist[1u + i], n, shift, SEG_STEPS_FAR);
+                    fixed |= seg_fix_run<K, V, DESC, true>(k, v, s_whist[1u + i], n, shift);
                 if (!__syncthreads_or((int)(fixed & (uint32_t)SEG_LONG))) return true;
             } else if (runs > 2047u) {
                 uint32_t fixed = 0;
-                for (uint32_t e = threadIdx.x; e < n; e += 8192u)
-                    fixed |= seg_fix_mask<K, V, DESC>(k, v, e, 256u, seg_tie_mask<K, DESC, false>(k, e, 256u, n, n, shift, inv), n, shift);
+                fixed = seg_fix_runs<K, V, DESC>(k, v, threadIdx.x, 256u, n, n, shift);
                 if (!__syncthreads_or((int)(fixed & (uint32_t)SEG_LONG))) return true;
             }
             return sorted(k, n);
