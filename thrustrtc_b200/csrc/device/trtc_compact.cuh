@@ -40,7 +40,7 @@ TRTC_FORCEINLINE T ld_view_nc(const V& v, size_t i) {
         const unsigned long long b = __ldg(reinterpret_cast<const unsigned long long*>(v._data + i));
         return *reinterpret_cast<const T*>(&b);
     } else {
-        return (T)v[i];
+        return (T)const_cast<V&>(v)[i];  // (a view's operator[] is not const)
     }
 }
 

@@ -13,7 +13,8 @@
 //     offsets keys by keys[TRTC_Min_Element], whose 256-wide tree (extrema.cpp:5-13 over
 //     internal/general_reduce.cpp:55-95) can select a non-minimum when NaNs sit in left slots;
 //     the sorted order is then a rotation, applied by the last digit pass's scatter;
-//   * short inputs: one CTA sorts all digits on chip in a single launch (radix_small_kernel);
+//   * short inputs: one CTA, or a cluster of 8 or 16, sorts all digits on chip in a single launch
+//     (radix_small_kernel);
 //   * one pass kernel per digit that moves data (the launches left over do nothing): a CTA takes tiles in launch order from an atomic counter,
 //     ranks its keys with warp multisplit (bit ballots), publishes per-digit counts,
 //     looks back across earlier tiles for its global offsets (decoupled look-back with
