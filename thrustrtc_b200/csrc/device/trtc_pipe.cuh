@@ -459,8 +459,9 @@ template <class K, class E, class T, int ITEMS, int S, int C> struct RbkSmem {
 
 // B200, 50,000,011 int32 keys in runs of mean 32 with float sums: 85-90 us per launch (4.4 TB/s,
 // 0.70 of the measured copy rate; segmented scan + tail compaction: 156 + 157 us); runs of 3:
-// 142 us, one run: 81 us.  Bound by issue (70 % busy, the ALU pipe 58 %): the fold of a tile costs
-// about 40 instructions per element.  Tiles of 20 elements per thread in 2 groups and 3 stages:
+// 142 us, one run: 81 us.  DRAM at 4.6 TB/s, issue 55 % busy, the ALU pipe 49 % (ncu): the fold of a tile
+// costs about 40 instructions per element.  Runs of one, 50 M: 467 us per call, bound by the ring, which
+// holds 1.5 tiles of results (two stages instead of three 275 us there, runs of 32 10 % slower).  Tiles of 20 elements per thread in 2 groups and 3 stages:
 // 87 us; 12 elements, 3 groups, 6 stages: 95 us; 12, 2, 6: 106 us (the per-tile part of the fold
 // spreads over fewer elements).  Two CTAs per SM of one group each, 12 elements: 128 us.
 //

@@ -347,9 +347,9 @@ TRTC_FORCEINLINE uint32_t radix_digit_sel(typename RadixKey<K>::B k, uint32_t se
     return DESC ? (d ^ 0xFFu) : d;
 }
 
-// Do the digit passes run as resident CTAs that take tile after tile?  Not of float keys: their passes are
-// bound by the instruction rate (three key codes per key and pass), and as a loop they lose more than
-// launches cost.  B200, us per sort, a CTA per tile against resident CTAs: 2^28 float keys 4646 / 4772,
+// Do the digit passes run as resident CTAs that take tile after tile?  Not of float keys: with
+// three key codes per key and pass theirs keep the load/store pipe 70 %, issue 66 % and the ALU pipe 60 %
+// busy, and as a loop they lose more than launches cost.  B200, us per sort, a CTA per tile against resident CTAs: 2^28 float keys 4646 / 4772,
 // descending 4655 / 4960, pairs 5623 / 5901; 30 M 592 / 602, pairs 709 / 733; 2^20 87 / 89, pairs 95 / 98.
 // (Doubles: 2^28 keys 15,623 / 15,071, pairs 18,122 / 17,546; u32 keys 4.54 / 4.36 ms, pairs 5.67 / 5.56.)
 template <class K> struct RadixResident { static constexpr bool value = !is_same<K, float>::value; };
